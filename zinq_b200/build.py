@@ -28,6 +28,10 @@ VARIANTS = [("line_inst.cu", f"line_{t[0]}{s}", [f"-DZQD_T={t}", f"-DZQD_S={s}",
 VARIANTS += [("nd_inst.cu", f"nd_{t[0]}{s}", [f"-DZQD_T={t}", f"-DZQD_S={s}", f"-DZQD_ND_CREATE=nd_create_{t[0]}{s}",
                                                f"-DZQD_ND_RUN=nd_run_{t[0]}{s}", f"-DZQD_ND_STEP=nd_step_{t[0]}{s}"])
              for t in ("double", "float") for s in (1, 2, 3, 4)]
+# the tile pass's kernels depend on the precision only
+VARIANTS += [("nd_tile.cu", f"nd_tile_{t[0]}", [f"-DZQD_T={t}", f"-DZQD_ND_TILE_PER_SM=nd_tile_per_sm_{t[0]}",
+                                                 f"-DZQD_ND_TILE_LAUNCH=nd_tile_launch_{t[0]}"])
+             for t in ("double", "float")]
 
 
 def _stale(target, deps):

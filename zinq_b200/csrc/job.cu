@@ -873,12 +873,12 @@ extern "C" int zqd_job_nd_shape(const zqd_job* J, zqd_nd_shape* out) {
     if (J->nd_row_tma) {
         out->tma_row_block = 1u << J->nd_row_tma_logL;
         out->tma_row_ctas = (uint32_t)J->nd_row_tma_ctas;
-        out->tma_row_threads = (uint32_t)((size_t)J->S * J->n * out->tma_row_block / 8);
+        out->tma_row_threads = (uint32_t)((size_t)J->S * J->n * out->tma_row_block / 16);
     }
     if (J->nd_tma) {
         out->tma_tile_lines = 1u << J->nd_tma_logW;
         out->tma_tile_ctas = (uint32_t)J->nd_tma_ctas;
-        out->tma_tile_threads = (uint32_t)((size_t)J->n * out->tma_tile_lines / 8);
+        out->tma_tile_threads = (uint32_t)((size_t)J->n * out->tma_tile_lines / 16);
     }
     out->rows_per_cta = (uint32_t)J->nd_rows;
     out->tile_lines = (uint32_t)J->nd_tile;

@@ -104,18 +104,17 @@ struct zqd_job {
     double min_gap = -1;                // ZQD_PRECISION_AUTO: smallest adiabatic gap on the grid (-1: not computed)
     int nd_rows = 1, nd_tile = 8, nd_row_threads = 32, nd_tile_threads = 32, nd_row_bufs = 2;
     // N-D strided-axis passes through the TMA-staged persistent kernel: lines per tile (log2), CTAs,
-    // and one tensor map (CUtensorMap, 128 bytes) over psi per strided axis
-    bool nd_tma = false;
+    // whether the stage and the exchange buffer share their space, and one tensor map (CUtensorMap,
+    // 128 bytes) over psi and over phi (the momentum passes) per strided axis
+    bool nd_tma = false, nd_tma_shared = true;
     int nd_tma_logW = 0, nd_tma_ctas = 0;
-    int nd_tma_ctas_full = 0; // the momentum-sum launches' grid: every resident CTA (never capped)
     alignas(64) unsigned char nd_maps[2][128] = {};
-    alignas(64) unsigned char nd_maps_phi[2][128] = {}; // the same over phi (the momentum passes)
-    // the row pass's TMA-staged persistent form: rows per block (log2), CTAs, tensor map over psi
-    bool nd_row_tma = false;
-    bool nd_row_tma_phi = false; // the momentum-copy launches too (else they take the earlier kernel)
-    int nd_row_tma_logL = 0, nd_row_tma_ctas = 0;
-    alignas(64) unsigned char nd_row_map[128] = {};
-    alignas(64) unsigned char nd_row_map_phi[128] = {}; // the same over phi (the momentum copy)
+    alignas(64) unsigned char nd_maps_phi[2][128] = {};
+    // the row pass's TMA-staged persistent form: rows per block (log2), CTAs of a launch without and
+    // with the momentum copy
+    bool nd_row_tma = false, nd_row_shared = true;
+    int nd_row_tma_logL = 0, nd_row_tma_ctas = 0, nd_row_phi_ctas = 0;
+    int nd_row_cols = 0, nd_k_cols = 0; // partial-sum columns of a row launch and of a momentum launch
     cudaGraphExec_t nd_graph = nullptr; // the whole N-D run, captured on its first call and replayed after
     bool nd_use_graph = true;           // false: launch directly (one-shot jobs skip the capture cost)
     float last_ms = 0;

@@ -11,6 +11,7 @@
 
 #include "job.h"
 #include "nd_kernels.cuh"
+#include "nd_tile.h"
 
 #if !defined(ZQD_T) || !defined(ZQD_S) || !defined(ZQD_ND_CREATE) || !defined(ZQD_ND_RUN) || !defined(ZQD_ND_STEP)
 #error "nd_inst.cu needs -DZQD_T, -DZQD_S, -DZQD_ND_CREATE, -DZQD_ND_RUN and -DZQD_ND_STEP"
@@ -66,6 +67,7 @@ NdJob<T> describe(zqd_job* J) {
     D.U = J->U.as<double>();
     D.capw = J->capw.as<double>();
     D.tw = J->tw.as<Tab<T>>();
+    D.twd = D.tw + J->n;
     D.kphase = J->expk.as<double2>();
     D.axis = reinterpret_cast<const double4*>(J->expk.as<double2>() + (size_t)J->d * J->n);
     D.part = J->part.as<double>();
@@ -85,54 +87,77 @@ NdJob<T> describe(zqd_job* J) {
 // and two 256-thread CTAs per SM hide more latency than extra registers would.
 inline bool row_narrow(unsigned threads) { return S > 1 && threads <= 256; }
 
-using RowTmaKernel = void (*)(NdJob<T>, CUtensorMap, CUtensorMap, NdRowTma, size_t, NdFin);
-// the momentum-copy form of the TMA row kernel (one state: with several it holds too many registers
-// for the per-block kernel's speed, and those launches take that kernel), or null
-inline RowTmaKernel row_tma_phi(int d) {
-    if constexpr (S == 1)
-        return d == 2 ? nd_row_tma_kernel<T, 2, S, true> : nd_row_tma_kernel<T, 3, S, true>;
-    else
+using RowTmaKernel = void (*)(NdJob<T>, NdRowTma, size_t, NdFin);
+// the longest line of the TMA-staged row pass: sixteen points a thread, at most 256 threads for the
+// states of one row, and no longer than the tile pass's
+constexpr int ROW_LOGN_MAX = S == 1 ? 12 : S == 2 ? 11 : 10;
+template <int D, int LOGN> RowTmaKernel row_tma_pick(int logn, int form) {
+    if constexpr (LOGN > ROW_LOGN_MAX || LOGN > nd_tma_logn_max<T>(D)) {
         return nullptr;
+    } else {
+        static const RowTmaKernel forms[RF_COUNT] = {
+            nd_row_tma_kernel<T, D, S, LOGN, RF_GENERAL>, nd_row_tma_kernel<T, D, S, LOGN, RF_POP>,
+            nd_row_tma_kernel<T, D, S, LOGN, RF_ACF>, nd_row_tma_kernel<T, D, S, LOGN, RF_ALL>};
+        return logn == LOGN ? forms[form] : row_tma_pick<D, LOGN + 1>(logn, form);
+    }
 }
-// the 512-thread plain form of the TMA row kernel (one or two states), or null
-inline RowTmaKernel row_tma_wide(int d) {
-    if constexpr (S <= 2)
-        return d == 2 ? nd_row_tma_kernel<T, 2, S, false, NDR_THREADS_WIDE> : nd_row_tma_kernel<T, 3, S, false, NDR_THREADS_WIDE>;
-    else
-        return nullptr;
+inline RowTmaKernel row_tma(int d, int logn, int form) {
+    return d == 2 ? row_tma_pick<2, ND_TMA_LOGN_MIN>(logn, form) : row_tma_pick<3, ND_TMA_LOGN_MIN>(logn, form);
 }
+inline int log2_of(int n) {
+    int l = 0;
+    while ((1 << l) < n) ++l;
+    return l;
+}
+// exchange line stride of the two passes (exch_stride): rows take consecutive threads; a tile's lines
+// sit side by side, as many as share a warp
+inline int row_ldx(int n) { return exch_stride<T>(log2_of(n), 0); }
+inline int tile_ldx(int n, int W) { return exch_stride<T>(log2_of(n), n <= 512 ? 512 / n : W); }
 
 struct Launch {
     zqd_job* J;
     NdJob<T> D;
     size_t nrow_blocks, ntile_blocks, ngrid;
+    size_t row_cols, k_cols; // partial-sum columns of a row launch and of a momentum launch
     // partial-sum regions (in blocks)
     size_t R0, R1, R2, K, G;
+    NdFin ahead{}; // sums waiting for the next tile launch's extra CTA (FIN_AHEAD), if enabled
+
+    // the waiting sums now, in a launch of their own
+    int flush() {
+        if (!ahead.enabled) return ZQD_OK;
+        nd_finalize_kernel<T><<<1, 256, 0, J->stream>>>(D, ahead);
+        ahead.enabled = 0;
+        ZQD_CUDA(cudaGetLastError());
+        return ZQD_OK;
+    }
 
     int row(uint32_t mode, uint32_t obs, size_t region, bool nostop = false, NdFin f = NdFin{}, cx<T>* wout = nullptr) {
         NdJob<T> d = D;
         d.wfn_out = wout;
         if (nostop) d.stopped = J->flags.as<int>() + 1; // a flag nothing sets
-        if (J->nd_row_tma && (!(mode & RM_PHI) || J->nd_row_tma_phi)) {
+        if (J->nd_row_tma) {
+            const bool phi = mode & RM_PHI;
             NdRowTma P{};
             P.mode = mode;
             P.obs = obs;
             P.logL = J->nd_row_tma_logL;
             P.nitems = (unsigned)(J->N / J->n >> P.logL);
+            P.workers = (unsigned)(phi ? J->nd_row_phi_ctas : J->nd_row_tma_ctas);
+            P.ncols = (unsigned)row_cols;
+            P.shared = phi || J->nd_row_shared;
+            P.ldx = row_ldx(J->n);
             bool withhold = false;
             P.wait_cycles = tma_wait_budget(NDT_WAIT_CYCLES, &withhold);
             P.withhold = withhold;
-            const size_t smem = ndr_smem_bytes<T>(S, 1 << P.logL, J->n);
-            const unsigned nt = (unsigned)((S * J->n << P.logL) / 8), nb = (unsigned)J->nd_row_tma_ctas;
-            const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(J->nd_row_map);
-            const CUtensorMap* mphi = reinterpret_cast<const CUtensorMap*>(J->nd_row_map_phi);
-            RowTmaKernel kern = D.d == 2 ? nd_row_tma_kernel<T, 2, S, false> : nd_row_tma_kernel<T, 3, S, false>;
-            if (!(obs & ~(uint32_t)(WM_POP | WM_NORM)) && nt <= (unsigned)NDR_THREADS) // populations and norm only
-                kern = D.d == 2 ? nd_row_tma_kernel<T, 2, S, false, NDR_THREADS, true>
-                                : nd_row_tma_kernel<T, 3, S, false, NDR_THREADS, true>;
-            if (mode & RM_PHI) kern = row_tma_phi(D.d); // only where nd_row_tma_phi (one state)
-            if (nt > (unsigned)NDR_THREADS) kern = row_tma_wide(D.d);
-            kern<<<nb, nt, smem, J->stream>>>(d, *map, *mphi, P, region, f);
+            const size_t smem = ndt_smem<T>(S << P.logL, J->n, P.ldx, P.shared, phi).total;
+            const unsigned nt = (unsigned)((S * J->n << P.logL) / 16);
+            int form = RF_ALL;
+            if (!(obs & ~row_form_obs(RF_POP))) form = RF_POP;
+            else if (!(obs & ~row_form_obs(RF_ACF))) form = RF_ACF;
+            if (d.track || d.wfn_out || (mode & RM_NORM)) form = RF_GENERAL;
+            const RowTmaKernel kern = row_tma(D.d, D.logn, form);
+            kern<<<P.workers, nt, smem, J->stream>>>(d, P, region, f);
             ZQD_CUDA(cudaGetLastError());
             return ZQD_OK;
         }
@@ -174,29 +199,32 @@ struct Launch {
         P.logtiles = logN - D.logn - P.logW;
         P.logO = logN - D.logn - lstride;
         P.nitems = (unsigned)S << P.logtiles;
-        P.ncols = (unsigned)(S * ntile_blocks); // the momentum region's width
-        const size_t smem = ndt_smem_bytes<T>(1 << P.logW, J->n);
-        const unsigned threads = (unsigned)((J->n << P.logW) / 8);
-        // the momentum sums are grouped per CTA: that launch's grid is the job's own (never the
-        // server's cap) and fits the region
-        const unsigned grid = (mode & TM_KOBS) ? (unsigned)std::min<size_t>((size_t)J->nd_tma_ctas_full, P.ncols)
-                                               : (unsigned)J->nd_tma_ctas;
+        P.shared = J->nd_tma_shared;
+        P.ldx = tile_ldx(J->n, 1 << P.logW);
+        const size_t smem = ndt_smem<T>(1 << P.logW, J->n, P.ldx, P.shared, false).total;
+        const unsigned threads = (unsigned)((J->n << P.logW) / 16);
+        P.workers = (unsigned)J->nd_tma_ctas;
+        if (phi) P.mode |= TM_PHI;
         bool withhold = false;
         P.wait_cycles = tma_wait_budget(NDT_WAIT_CYCLES, &withhold);
         P.withhold = withhold;
-        if (D.d == 2) nd_tile_tma_kernel<T, 2><<<grid, threads, smem, J->stream>>>(d, *map, P, region, f);
-        else nd_tile_tma_kernel<T, 3><<<grid, threads, smem, J->stream>>>(d, *map, P, region, f);
-        ZQD_CUDA(cudaGetLastError());
-        return ZQD_OK;
+        return nd_tile_launch<T>(D.logn, d, *map, P, region, f, P.workers + (f.enabled == FIN_AHEAD), threads, smem, J->stream);
     }
-    int ptile(int axis, uint32_t mode) { return J->nd_tma ? tile_tma(axis, mode) : tile(axis, mode, 0); }
-    // forward along axes d-2..1, forward + kinetic phase + inverse along axis 0, inverse along 1..d-2;
-    // `first`: mode bits of the first of these launches only (TM_SCALE)
-    int step_tiles(uint32_t first = 0) {
+    int ptile(int axis, uint32_t mode) {
+        if (!J->nd_tma) {
+            const int rc = flush();
+            return rc ? rc : tile(axis, mode, 0);
+        }
+        const NdFin f = ahead;
+        ahead.enabled = 0;
+        return tile_tma(axis, mode, false, 0, false, f);
+    }
+    // forward along axes d-2..1, forward + kinetic phase + inverse along axis 0, inverse along 1..d-2
+    int step_tiles() {
         int rc;
-        for (int a = D.d - 2; a >= 1; --a, first = 0)
-            if ((rc = ptile(a, TM_FWD | first))) return rc;
-        if ((rc = ptile(0, TM_FWD | TM_KPHASE | TM_INV | first))) return rc;
+        for (int a = D.d - 2; a >= 1; --a)
+            if ((rc = ptile(a, TM_FWD))) return rc;
+        if ((rc = ptile(0, TM_FWD | TM_KPHASE | TM_INV))) return rc;
         for (int a = 1; a <= D.d - 2; ++a)
             if ((rc = ptile(a, TM_INV))) return rc;
         return ZQD_OK;
@@ -239,41 +267,44 @@ struct Launch {
     }
 };
 
-// resident CTAs per SM the tile pass's persistent grid may use: the job server's setting, else
-// all that fit (the tile pass reduces nothing, so its grid changes no result)
-inline int tma_ctas_per_sm_cap(const zqd_job* J) { return J->o.tma_ctas_per_sm > 0 ? J->o.tma_ctas_per_sm : 1 << 20; }
+// Grid of a persistent pass: with room for every item at once the stage and the exchange buffer share
+// their space (more CTAs fit); otherwise they are separate, so that a CTA's next load overlaps its work,
+// where that still leaves two CTAs per SM.  per_sm(smem): resident CTAs per SM; extra: CTAs of the
+// launch that take no items (they must not wait for a worker to leave).
+template <typename F>
+int choose_grid(size_t items, int sms, int extra, size_t smem_shared, size_t smem_apart, const F& per_sm, bool& shared,
+                int& ctas) {
+    int a = 0, b = 0, rc;
+    if ((rc = per_sm(smem_shared, &a))) return rc;
+    shared = true;
+    if (items > (size_t)a * sms && smem_apart <= (size_t)ND_SMEM_BUDGET) {
+        if ((rc = per_sm(smem_apart, &b))) return rc;
+        if (b >= 2) shared = false;
+    }
+    ctas = (int)std::min<size_t>(items, (size_t)std::max(1, shared ? a : b) * sms - (size_t)extra);
+    return ZQD_OK;
+}
 
 // The TMA-staged tile pass: lines per tile W (a power of two, W <= n) with rows of W c >= 16
-// bytes (an even number of 8-byte words), W n / 8 threads (whole warps, at most 512) and two
-// stages within the shared-memory budget; by default the widest W up to 64-byte rows.  w_override
+// bytes (an even number of 8-byte words), W n / 16 threads (whole warps, at most 256, 512 on lines of
+// 4096 points; a line of at most 512 points within one warp) and the stage, exchange and
+// twiddles within the shared-memory budget; by default the widest W up to 64-byte rows.  w_override
 // (the autotuner's candidate or table entry): 0 keeps the default, -1 keeps the earlier tile
 // kernel, else W.  ZQD_ND_TMA=0 in the environment also keeps it.
-int setup_tma(zqd_job* J, int w_override) {
+int setup_tma_shape(zqd_job* J, int w_override) {
     constexpr int c = (int)sizeof(cx<T>), E = c / 8;
-    const int n = J->n, d = J->d;
-    const size_t budget = 200 * 1024;
+    const int n = J->n, d = J->d, logn = log2_of(n);
     J->nd_tma = false;
     const char* env = getenv("ZQD_ND_TMA");
-    if ((env && env[0] == '0') || w_override < 0) return ZQD_OK;
+    if ((env && env[0] == '0') || w_override < 0 || logn < ND_TMA_LOGN_MIN || logn > nd_tma_logn_max<T>(d)) return ZQD_OK;
     int dev = 0, sms = 148;
     ZQD_CUDA(cudaGetDevice(&dev));
     ZQD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    for (auto f : {nd_tile_tma_kernel<T, 2>, nd_tile_tma_kernel<T, 3>})
-        ZQD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    const size_t tmax = logn == 12 ? 512 : 256;
     auto fits = [&](int W) {
-        return W >= 1 && W <= n && (E * W) % 2 == 0 && (size_t)W * n / 8 <= 512 && ((size_t)W * n / 8) % 32 == 0 &&
-               ndt_smem_bytes<T>(W, n) <= budget;
-    };
-    // resident CTAs on the device for a W (the job's own count: the shape, and with it every result,
-    // must not depend on the server's cap, which only trims the grid of the passes that sum nothing)
-    auto ctas_for = [&](int W, int& ctas) -> int {
-        const int threads = W * n / 8;
-        int per_sm = 0;
-        ZQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, d == 2 ? (const void*)nd_tile_tma_kernel<T, 2> : (const void*)nd_tile_tma_kernel<T, 3>, threads,
-            ndt_smem_bytes<T>(W, n)));
-        ctas = std::max(1, per_sm) * sms;
-        return ZQD_OK;
+        const size_t t = (size_t)W * n / 16;
+        return W >= 1 && W <= n && (E * W) % 2 == 0 && t <= tmax && t % 32 == 0 &&
+               ndt_smem<T>(W, n, tile_ldx(n, W), true, false).total <= (size_t)ND_SMEM_BUDGET;
     };
     const size_t lines = J->N / (size_t)n; // lines of one state along any axis
     int W = 0;
@@ -281,24 +312,28 @@ int setup_tma(zqd_job* J, int w_override) {
     if (W) {
         if (!fits(W) || lines % (size_t)W) return fail(ZQD_ERR_UNSUPPORTED, "TMA TILE SHAPE OUTSIDE THE KERNEL'S LIMITS");
     } else {
-        // measured: 32- to 64-byte rows win; on 2-D FP32 lines of 512 points 32-byte rows (twice the
-        // tiles) were 3-5 % faster per step than 64-byte rows with 1 to 3 states
-        const int wmax = (c == 8 && d == 2 && n == 512) ? 32 / c : 64 / c;
-        for (int w = std::max(1, wmax); w >= 1 && !W; w >>= 1)
-            if (fits(w) && lines % (size_t)w == 0) W = w;
+        // 64-byte rows, or 32-byte rows where that gives the device fewer than two tiles per SM (and the
+        // lines of one warp where those are more)
+        for (int w = std::max(64 / c, 512 / n); w >= 1 && !W; w >>= 1)
+            if (fits(w) && lines % (size_t)w == 0 && (w * c <= 32 || (size_t)S * (lines / w) >= 2 * (size_t)sms || !fits(w / 2))) W = w;
         if (!W) return ZQD_OK; // no shape fits: the earlier tile kernel runs
     }
-    int logW = 0;
-    while ((1 << logW) < W) ++logW;
-    int ctas = 0, rc;
-    if ((rc = ctas_for(W, ctas))) return rc;
     const size_t items = (size_t)S * (lines / W);
-    J->nd_tma_ctas_full = (int)std::min<size_t>(items, (size_t)ctas);
-    const int per_sm = ctas / sms;
-    J->nd_tma_ctas = (int)std::min<size_t>(items, (size_t)std::min(per_sm, tma_ctas_per_sm_cap(J)) * sms);
-    J->nd_tma_logW = logW;
-    int logn = 0;
-    while ((1 << logn) < n) ++logn;
+    const int ldx = tile_ldx(n, W);
+    int rc;
+    if ((rc = choose_grid(items, sms, 1, ndt_smem<T>(W, n, ldx, true, false).total, ndt_smem<T>(W, n, ldx, false, false).total,
+                          [&](size_t smem, int* per) { return nd_tile_per_sm<T>(d, logn, W * n / 16, smem, per); },
+                          J->nd_tma_shared, J->nd_tma_ctas)))
+        return rc;
+    J->nd_tma_logW = log2_of(W);
+    J->nd_tma = true;
+    return ZQD_OK;
+}
+
+// the tile pass's tensor maps over psi and phi, one per strided axis (after they are allocated)
+int encode_tile_maps(zqd_job* J) {
+    constexpr int c = (int)sizeof(cx<T>), E = c / 8;
+    const int n = J->n, d = J->d, logn = log2_of(n), W = 1 << J->nd_tma_logW;
     for (int a = 0; a + 1 < d; ++a) {
         const int lstride = logn * (d - 1 - a);
         const uint64_t st = (uint64_t)1 << lstride, O = J->N / ((uint64_t)n * st);
@@ -311,87 +346,54 @@ int setup_tma(zqd_job* J, int w_override) {
                                     (uint64_t)n * st * c, box, l2);
         if (e) return fail(ZQD_ERR_DEVICE, "cuTensorMapEncodeTiled failed for the tile pass");
     }
-    J->nd_tma = true;
     return ZQD_OK;
 }
 
-// The TMA-staged row pass: L rows (a power of two dividing N/n) per block with L n c >= 1024 bytes
-// (the stages keep the 128-byte swizzle's 1024-byte alignment), S L n / 8 threads (whole warps, at
-// most 256, or 512 for one or two states on lines too long for 256; the momentum copy then takes
-// the per-block kernel) and two stages within the budget; by default the largest L of at most 256
-// threads (the wide form only where no 256-thread block fits).  The grid takes every resident CTA
-// (jobs created by the server too: its observables' sums are grouped per CTA, so a job's results
-// depend on its grid, which must not change with where it runs).
-// l_override: 0 keeps the default, -1 keeps the earlier row kernel, else L.  ZQD_ND_TMA=0 also
-// keeps it.
+// The TMA-staged row pass: L rows (a power of two dividing N/n) per block, S L n / 16 threads (whole
+// warps, at most 256) and the stage, exchange (and, for the momentum copy, its lines) and twiddles
+// within the budget.  The grid takes every resident CTA (jobs created by the server too: its
+// observables' sums are grouped per CTA, so a job's results depend on its grid, which must not change
+// with where it runs).  l_override: 0 keeps the default, -1 keeps the earlier row kernel, else L.
+// ZQD_ND_TMA=0 also keeps it.
 int choose_row_tma(zqd_job* J, int l_override) {
-    constexpr int c = (int)sizeof(cx<T>);
-    const int n = J->n, d = J->d;
-    const size_t budget = 200 * 1024, lines = J->N / (size_t)n;
+    const int n = J->n, d = J->d, logn = log2_of(n), ldx = logn >= ND_TMA_LOGN_MIN ? row_ldx(n) : n;
+    const size_t lines = J->N / (size_t)n;
     J->nd_row_tma = false;
     const char* env = getenv("ZQD_ND_TMA");
-    if ((env && env[0] == '0') || l_override < 0) return ZQD_OK;
+    if ((env && env[0] == '0') || l_override < 0 || logn < ND_TMA_LOGN_MIN || !row_tma(d, logn, RF_GENERAL)) return ZQD_OK;
     int dev = 0, sms = 148;
     ZQD_CUDA(cudaGetDevice(&dev));
     ZQD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    for (auto f : {nd_row_tma_kernel<T, 2, S, false>, nd_row_tma_kernel<T, 3, S, false>,
-                   nd_row_tma_kernel<T, 2, S, false, NDR_THREADS, true>, nd_row_tma_kernel<T, 3, S, false, NDR_THREADS, true>})
-        ZQD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
-    for (int dd : {2, 3})
-        for (RowTmaKernel f : {row_tma_wide(dd), row_tma_phi(dd)})
-            if (f) ZQD_CUDA(cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
-    auto threads_of = [&](int L) { return (size_t)S * L * n / 8; };
+    for (int form = 0; form < RF_COUNT; ++form)
+        ZQD_CUDA(cudaFuncSetAttribute((const void*)row_tma(d, logn, form), cudaFuncAttributeMaxDynamicSharedMemorySize, ND_SMEM_BUDGET));
+    auto threads_of = [&](int L) { return (size_t)S * L * n / 16; };
     auto fits = [&](int L) {
         const size_t t = threads_of(L);
-        // whole warps: the block reduction's shuffles run on full warps
-        return L >= 1 && (size_t)L <= lines && lines % (size_t)L == 0 && (size_t)L * n * c >= 1024 && t % 32 == 0 &&
-               (t <= (size_t)NDR_THREADS || (t <= (size_t)NDR_THREADS_WIDE && row_tma_wide(d))) &&
-               ndr_smem_bytes<T>(S, L, n) <= budget;
-    };
-    auto ctas_for = [&](int L, int& ctas) -> int {
-        const unsigned nt = (unsigned)threads_of(L);
-        const void* f = nt > (unsigned)NDR_THREADS ? (const void*)row_tma_wide(d)
-                        : d == 2                   ? (const void*)nd_row_tma_kernel<T, 2, S, false>
-                                                   : (const void*)nd_row_tma_kernel<T, 3, S, false>;
-        int per_sm = 0;
-        ZQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, (int)nt, ndr_smem_bytes<T>(S, L, n)));
-        ctas = std::max(1, per_sm) * sms;
-        return ZQD_OK;
+        return L >= 1 && (size_t)L <= lines && lines % (size_t)L == 0 && t % 32 == 0 && t <= (size_t)NDR_THREADS &&
+               ndt_smem<T>(S * L, n, ldx, true, true).total <= (size_t)ND_SMEM_BUDGET;
     };
     int L = 0;
     if (l_override > 0) L = l_override;
     if (L) {
         if (!fits(L)) return fail(ZQD_ERR_UNSUPPORTED, "TMA ROW-BLOCK SHAPE OUTSIDE THE KERNEL'S LIMITS");
-    } else { // the largest block of at most 256 threads (measured: fewer, larger CTAs win), else the wide form
-        for (int l = std::max(1, 4096 / (S * n)); l >= 1 && !L; l >>= 1)
-            if (fits(l) && (threads_of(l) <= (size_t)NDR_THREADS || !fits(l / 2))) L = l;
+    } else { // the smallest block of at least 64 threads
+        for (int l = 1; (size_t)l <= lines && !L; l <<= 1)
+            if (fits(l) && (threads_of(l) >= 64 || !fits(2 * l))) L = l;
         if (!L) return ZQD_OK; // no shape fits: the earlier row kernel runs
     }
-    int logL = 0;
-    while ((1 << logL) < L) ++logL;
-    int ctas = 0, rc;
-    if ((rc = ctas_for(L, ctas))) return rc;
-    J->nd_row_tma_ctas = (int)std::min<size_t>(lines / L, (size_t)ctas);
-    J->nd_row_tma_logL = logL;
-    // the momentum-copy form holds the end-of-step state in registers besides the sweep's: with one
-    // state it keeps up with the per-block kernel, with several it does not (one CTA per SM)
-    J->nd_row_tma_phi = row_tma_phi(d) && threads_of(L) <= (size_t)NDR_THREADS;
+    int rc;
+    bool shared_phi = true;
+    const size_t phi_smem = ndt_smem<T>(S * L, n, ldx, true, true).total; // the momentum copy always shares
+    auto per_sm = [&](size_t smem, int* per) -> int {
+        ZQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, (const void*)row_tma(d, logn, RF_ALL), (int)threads_of(L), smem));
+        return ZQD_OK;
+    };
+    if ((rc = choose_grid(lines / L, sms, 0, ndt_smem<T>(S * L, n, ldx, true, false).total,
+                          ndt_smem<T>(S * L, n, ldx, false, false).total, per_sm, J->nd_row_shared, J->nd_row_tma_ctas)) ||
+        (rc = choose_grid(lines / L, sms, 0, phi_smem, (size_t)ND_SMEM_BUDGET + 1, per_sm, shared_phi, J->nd_row_phi_ctas)))
+        return rc;
+    J->nd_row_tma_logL = log2_of(L);
     J->nd_row_tma = true;
-    return ZQD_OK;
-}
-
-// the row pass's tensor maps over psi and phi (after they are allocated)
-int encode_row_tma(zqd_job* J) {
-    constexpr int c = (int)sizeof(cx<T>);
-    const int L = 1 << J->nd_row_tma_logL, n = J->n;
-    const uint64_t rows_total = (uint64_t)S * J->N * c / 128;
-    const uint64_t dims[3] = {16, rows_total, 1};
-    const uint32_t box[3] = {16, (uint32_t)std::min<uint64_t>(256, (uint64_t)L * n * c / 128), 1};
-    if (encode_map_3d(reinterpret_cast<CUtensorMap*>(J->nd_row_map), J->psi_save.p, dims, 128, rows_total * 128, box, 256,
-                      true) ||
-        encode_map_3d(reinterpret_cast<CUtensorMap*>(J->nd_row_map_phi), J->phi.p, dims, 128, rows_total * 128, box, 256,
-                      true))
-        return fail(ZQD_ERR_DEVICE, "cuTensorMapEncodeTiled failed for the row pass");
     return ZQD_OK;
 }
 
@@ -406,7 +408,7 @@ int ZQD_ND_CREATE(zqd_job* J) {
     // buffers; one thread per 8-point group).
     // Tile pass: Tn lines per CTA, rows of Tn * c >= 32 bytes (one sector), shrunk from
     // 128 bytes until the grid has two CTAs per SM.
-    const int budget = 200 * 1024, sms2 = 2 * 148;
+    const int budget = ND_SMEM_BUDGET, sms2 = 2 * 148;
     const int max_items = 512; // 8-point groups of a CTA, one thread each
     J->nd_row_bufs = 2;
     if (S * n > 8 * max_items) return fail(ZQD_ERR_UNSUPPORTED, "GRID LINE TOO LONG FOR THE ROW PASS (states x npoint at most 4096)");
@@ -444,21 +446,11 @@ int ZQD_ND_CREATE(zqd_job* J) {
     }
     J->nd_tile_threads = std::max(32, (Tn * n / 8 + 31) / 32 * 32);
     int rc;
-    // The TMA-staged row pass, where a shape fits: the per-block row kernel (the launches the TMA
-    // form does not take) uses the same rows per block, so both write every column of a partial-sum
-    // region, one column per block.
-    if ((rc = choose_row_tma(J, ov.tma_rows))) return rc;
-    if (J->nd_row_tma) {
-        const int Lt = 1 << J->nd_row_tma_logL;
-        if (S * Lt * n / 8 <= max_items && nd_smem_bytes<T>(J->nd_row_bufs, S * Lt, n) <= (size_t)budget) {
-            J->nd_rows = L = Lt;
-            J->nd_row_threads = std::max(32, (S * L * n / 8 + 31) / 32 * 32);
-        } else {
-            J->nd_row_tma = false;
-        }
-    }
-    const size_t nrow_blocks = N / n / L, ntile_blocks = N / n / Tn;
-    const size_t nparts = 3 * nrow_blocks + S * ntile_blocks + 1024;
+    if ((rc = choose_row_tma(J, ov.tma_rows)) || (rc = setup_tma_shape(J, ov.tma_w))) return rc;
+    // columns of the partial sums: one per CTA of a row launch or of a momentum launch
+    J->nd_row_cols = J->nd_row_tma ? std::max(J->nd_row_tma_ctas, J->nd_row_phi_ctas) : (int)(N / n / L);
+    J->nd_k_cols = J->nd_tma ? J->nd_tma_ctas : (int)(S * (N / n / Tn));
+    const size_t nparts = 3 * (size_t)J->nd_row_cols + J->nd_k_cols + 1024;
     if ((rc = J->psi_save.alloc((size_t)S * N * c, J->stream))) return rc;
     if ((rc = J->phi.alloc((size_t)S * N * c, J->stream))) return rc;
     if ((o.has_spectrum || (o.write_mask & ZQD_WRITE_ACF)) && (rc = J->psi0.alloc((size_t)S * N * c, J->stream))) return rc;
@@ -467,7 +459,7 @@ int ZQD_ND_CREATE(zqd_job* J) {
     if ((rc = J->V.alloc((size_t)S * S * N * sizeof(double), J->stream))) return rc;
     if (S > 1 && (rc = J->U.alloc((size_t)S * S * N * sizeof(double), J->stream))) return rc;
     if (o.has_cap && (rc = J->capw.alloc(N * sizeof(double), J->stream))) return rc;
-    if ((rc = J->tw.alloc((size_t)n * tb, J->stream))) return rc;
+    if ((rc = J->tw.alloc((size_t)2 * n * tb, J->stream))) return rc; // natural order, then pass by pass
     if ((rc = J->expk.alloc((size_t)J->d * n * (sizeof(double2) + sizeof(double4)), J->stream))) return rc; // phases, axis table
     if ((rc = J->part.alloc(nparts * NDV * 2 * sizeof(double), J->stream))) return rc;
     if ((o.write_mask & ZQD_WRITE_WAVEFUNCTION) &&
@@ -490,12 +482,13 @@ int ZQD_ND_CREATE(zqd_job* J) {
     J->device_bytes = J->psi_save.bytes + J->phi.bytes + J->psi0.bytes + J->orth.bytes + J->R.bytes + J->V.bytes +
                       J->U.bytes + J->capw.bytes + J->part.bytes + J->hist.bytes;
     std::vector<double> tw = twiddles_f64(n);
-    std::vector<Tab<T>> twt(n);
+    std::vector<Tab<T>> twt(2 * (size_t)n);
     for (int t = 0; t < n; ++t) twt[t] = mktab<T>(tw[2 * t], tw[2 * t + 1]);
-    ZQD_CUDA(cudaMemcpyAsync(J->tw.p, twt.data(), (size_t)n * tb, cudaMemcpyHostToDevice, J->stream));
+    dense_twiddles(log2_of(n), twt.data(), twt.data() + n);
+    ZQD_CUDA(cudaMemcpyAsync(J->tw.p, twt.data(), 2 * (size_t)n * tb, cudaMemcpyHostToDevice, J->stream));
     ZQD_CUDA(cudaMemsetAsync(J->flags.p, 0, 4 * sizeof(int), J->stream));
     ZQD_CUDA(cudaMemsetAsync(J->hist.p, 0xff, J->hist.bytes, J->stream)); // NaN until written
-    J->h2d += (size_t)n * tb + J->pot.bytes;
+    J->h2d += 2 * (size_t)n * tb + J->pot.bytes;
     NdJob<T> D = describe(J);
     nd_table_kernel<T, S><<<(unsigned)((N + 127) / 128), 128, 0, J->stream>>>(D, 0.0, 1);
     ZQD_CUDA(cudaGetLastError());
@@ -507,8 +500,7 @@ int ZQD_ND_CREATE(zqd_job* J) {
         ZQD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
     for (auto f : {nd_tile_kernel<T, 2>, nd_tile_kernel<T, 3>})
         ZQD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-    if ((rc = setup_tma(J, ov.tma_w))) return rc;
-    if (J->nd_row_tma && (rc = encode_row_tma(J))) return rc;
+    if (J->nd_tma && (rc = encode_tile_maps(J))) return rc;
     ZQD_CUDA(cudaStreamSynchronize(J->stream));
     return ZQD_OK;
 }
@@ -532,11 +524,13 @@ struct Seq {
         Lc.nrow_blocks = N / J->n / J->nd_rows;
         Lc.ntile_blocks = N / J->n / J->nd_tile;
         Lc.ngrid = std::min<size_t>(1024, (N + 255) / 256);
+        Lc.row_cols = (size_t)J->nd_row_cols;
+        Lc.k_cols = (size_t)J->nd_k_cols;
         Lc.R0 = 0;
-        Lc.R1 = Lc.nrow_blocks;
-        Lc.R2 = 2 * Lc.nrow_blocks;
-        Lc.K = 3 * Lc.nrow_blocks;
-        Lc.G = Lc.K + S * Lc.ntile_blocks;
+        Lc.R1 = Lc.row_cols;
+        Lc.R2 = 2 * Lc.row_cols;
+        Lc.K = 3 * Lc.row_cols;
+        Lc.G = Lc.K + Lc.k_cols;
         split = o.imag_nstate > 0 || o.pot_td || (o.has_cap && o.cap_has_stop);
         acf = o.has_spectrum || (o.write_mask & ZQD_WRITE_ACF);
         iters = (int)o.iterations;
@@ -553,8 +547,8 @@ struct Seq {
     // positions are quadratic in psi and the autocorrelation is linear, so the step closes and the
     // next one opens in a single row pass over the unnormalised psi, as in real time; its finalize
     // scales the observables row by the renormalisation factor (squared) and keeps the sum of
-    // |psi|^2, and the first tile pass of step i+1 (or the final observables' pass) multiplies psi
-    // by that factor as it loads it.
+    // |psi|^2, and the row pass that closes step i+1 (or the final observables' pass) multiplies psi
+    // by that factor.
     bool deferred(int s) const {
         const Opts& o = J->o;
         return o.imag_nstate && s == 0 && !o.has_cap && !o.pot_td && !J->wfn_hist.p;
@@ -573,13 +567,13 @@ struct Seq {
         f.x0 = x0;
         f.x1 = x1;
         f.k0 = Lc.K;
-        f.k1 = k ? Lc.K + S * Lc.ntile_blocks : Lc.K;
+        f.k1 = k ? Lc.K + Lc.k_cols : Lc.K;
         f.stop_norm = o.cap_stop_norm;
         f.mask = mask;
         f.row_index = i;
         f.kind = kind;
         f.has_stop = kind == 0 && o.has_cap && o.cap_has_stop;
-        f.enabled = 1;
+        f.enabled = FIN_LAST;
         return f;
     }
     int itp_ops(int s) { // quantum_dynamics.zig:898-906
@@ -620,16 +614,18 @@ struct Seq {
         const uint32_t obs = mask | ((o.has_cap && o.cap_has_stop) ? (uint32_t)WM_NORM : 0u);
         double* row = hist(s) + (size_t)i * HC;
         const bool defer = deferred(s);
-        if (i > 0 && (rc = Lc.step_tiles(defer ? (uint32_t)TM_SCALE : 0u))) return rc;
+        if (i > 0 && (rc = Lc.step_tiles())) return rc;
         if (!split || defer) {
             uint32_t mode = RM_OBS | RM_STORE | (needk ? RM_PHI : 0u);
-            if (i > 0) mode |= RM_INV | RM_REND;
+            if (i > 0) mode |= RM_INV | RM_REND | (defer ? (uint32_t)RM_SCALE : 0u);
             if (i < iters) mode |= RM_RSTART | RM_FWD;
-            NdFin f = fin(s, 0, Lc.R0, Lc.R0 + Lc.nrow_blocks, needk, mask, row, i);
+            NdFin f = fin(s, 0, Lc.R0, Lc.R0 + Lc.row_cols, needk, mask, row, i);
             if (defer) f.nsum_out = Lc.scal();
             const uint32_t o2 = obs | (defer ? (uint32_t)WM_NORM : 0u);
-            if ((rc = Lc.row(mode, o2, Lc.R0, false, needk ? NdFin{} : f, whist(s, i)))) return rc;
-            if (needk && (rc = Lc.kobs(false, f))) return rc;
+            if ((rc = Lc.row(mode, o2, Lc.R0, false, NdFin{}, whist(s, i)))) return rc;
+            if (needk && (rc = Lc.kobs(false, NdFin{}))) return rc;
+            f.enabled = FIN_AHEAD; // by the next step's first tile launch
+            Lc.ahead = f;
             return ZQD_OK;
         }
         // Imaginary time, first state (nothing to orthogonalise against), no absorbing potential, after
@@ -640,13 +636,13 @@ struct Seq {
         const bool fuse = o.imag_nstate && s == 0 && i > 0 && !o.has_cap;
         if (i > 0 && (rc = Lc.row(RM_INV | RM_REND | RM_STORE | (fuse ? (uint32_t)RM_NORM : 0u), 0, Lc.R0))) return rc;
         if (fuse) { // the norm's sum into scal[0], taken out of R0 (the observables row sums R0 too)
-            if ((rc = Lc.reduce(Lc.R0, Lc.R0 + Lc.nrow_blocks, 1, true))) return rc;
+            if ((rc = Lc.reduce(Lc.R0, Lc.R0 + Lc.row_cols, 1, true))) return rc;
         } else if (o.imag_nstate && (rc = itp_ops(s))) {
             return rc; // every i, the initial state included
         }
         if (o.pot_td && (rc = Lc.table((double)i * o.time_step, 0))) return rc;
         // R0 holds the end-of-step sums of the row pass that closed step i (none at i = 0)
-        const NdFin f = fin(s, 0, i > 0 ? Lc.R0 : Lc.R1, Lc.R1 + Lc.nrow_blocks, needk, mask, row, i);
+        const NdFin f = fin(s, 0, i > 0 ? Lc.R0 : Lc.R1, Lc.R1 + Lc.row_cols, needk, mask, row, i);
         if (fuse && !o.pot_td && i < iters) { // normalise, observe, and open step i+1 in one pass
             const uint32_t mode = RM_SCALE | RM_OBS | RM_RSTART | RM_FWD | RM_STORE | (needk ? (uint32_t)RM_PHI : 0u);
             if ((rc = Lc.row(mode, obs, Lc.R1, false, needk ? NdFin{} : f, whist(s, i)))) return rc;
@@ -659,19 +655,20 @@ struct Seq {
         if (i < iters) {
             if (o.pot_td && (rc = Lc.table(((double)i + 0.5) * o.time_step, 1))) return rc;
             // the absorbed sums of step i+1's first accumAbsorbed
-            const NdFin fc = fin(s, 2, Lc.R2, Lc.R2 + Lc.nrow_blocks, false, 0, nullptr, 0);
+            const NdFin fc = fin(s, 2, Lc.R2, Lc.R2 + Lc.row_cols, false, 0, nullptr, 0);
             if ((rc = Lc.row(RM_RSTART | RM_FWD | RM_STORE, 0, Lc.R2, false, fc))) return rc;
         }
         return ZQD_OK;
     }
     int epilogue(int s) {
         int rc;
+        if ((rc = Lc.flush())) return rc;
         // final Observables.init(..., log = true) (quantum_dynamics.zig:949)
         const uint32_t all = WM_ALL_OBS | (acf ? (uint32_t)WM_ACF : 0u);
         // a deferred renormalisation (the last step's) is applied here, and psi stored normalised
         const uint32_t scale = deferred(s) ? (uint32_t)(RM_SCALE | RM_STORE) : 0u;
         if ((rc = Lc.row(RM_OBS | RM_PHI | scale, all, Lc.R1, true))) return rc;
-        if ((rc = Lc.kobs(true, fin(s, 1, Lc.R1, Lc.R1 + Lc.nrow_blocks, true, all, J->fin.as<double>() + (size_t)s * HC, 0))))
+        if ((rc = Lc.kobs(true, fin(s, 1, Lc.R1, Lc.R1 + Lc.row_cols, true, all, J->fin.as<double>() + (size_t)s * HC, 0))))
             return rc;
         if (s + 1 < J->nsolve) // orthw.append (quantum_dynamics.zig:586-591)
             ZQD_CUDA(cudaMemcpyAsync(J->orth.as<char>() + (size_t)s * SN, J->psi_save.p, SN, cudaMemcpyDeviceToDevice, J->stream));
@@ -713,6 +710,7 @@ int ZQD_ND_STEP(zqd_job* J, int s, int i0, int i1, int* rows, int* ended) {
     if (i0 == 0 && (rc = q.prologue(s))) return rc;
     for (int i = i0; i <= i1; ++i)
         if ((rc = q.step(s, i))) return rc;
+    if ((rc = q.Lc.flush())) return rc;
     // the steps first, then the copies into pageable memory (one queued behind the steps would wait
     // inside the driver, where it can hold up other threads' copies)
     ZQD_CUDA(cudaStreamSynchronize(J->stream));

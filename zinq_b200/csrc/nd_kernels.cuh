@@ -18,14 +18,18 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "cx.cuh"
 #include "line_kernel.cuh"
+#include "nd_fft.cuh"
 #include "physics.cuh"
 #include "tma.cuh"
 
 namespace zqd {
 
 constexpr int NDV = 24; // reduction slots of the N-D passes
+constexpr int ND_SMEM_BUDGET = 200 * 1024; // dynamic shared memory of a CTA
 
 // norm | pos[d] | epot | acf re, im | mom[d] | ekin | pop[S] | absorbed, this step [S] | absorbed, next step [S]
 struct NdSlots {
@@ -61,6 +65,7 @@ template <typename T> struct NdJob {
     double* U;    // [S*S][N]
     double* capw; // [N]
     const Tab<T>* tw; // [n] exp(-2 pi i t / n)
+    const Tab<T>* twd; // the same pass by pass for the TMA-staged passes (LinePlan's dense table)
     const double2* kphase; // [D][n] exp(Complex(0, -k^2 / (2 m_j)) * dt) of axis j
     const double4* axis;   // [D][n] per-axis grid values: coordinate r, wavenumber k, 0.5 k^2 / m_j
     double* part;     // per-CTA partial sums, slot-major: [NDV][nparts][2]
@@ -83,7 +88,7 @@ enum : uint32_t {
     RM_FWD = 1u << 5,    // forward FFT along the last axis
     RM_STORE = 1u << 6,  // write psi back
     RM_NORM = 1u << 7,   // after RM_REND: sum |psi|^2 into the norm slot (imaginary time: the renormalisation's norm)
-    RM_SCALE = 1u << 8,  // on load: psi /= sqrt(dr * *nsum), as the normalisation kernel does (imaginary time)
+    RM_SCALE = 1u << 8,  // after the inverse transform: psi *= nd_norm_factor(*nsum, dr) (imaginary time)
 };
 // tile-pass modes
 enum : uint32_t {
@@ -92,7 +97,6 @@ enum : uint32_t {
     TM_INV = 1u << 2,
     TM_KOBS = 1u << 3,   // after the forward FFT along axis 0: momentum observables, no store
     TM_PHI = 1u << 4,    // operate on phi instead of psi
-    TM_SCALE = 1u << 5,  // on load: psi *= nd_norm_factor(*nsum, dr) (imaginary time, renormalisation deferred)
 };
 
 // The renormalisation factor of psi whose sum of |psi|^2 is `sum`: 1 / sqrt(dr * sum), formed as
@@ -307,7 +311,11 @@ struct NdBook {
     unsigned counter; // CTAs of the current launch that have written their partials
 };
 
-// What the last CTA of a row or tile launch does with the partial sums (enabled != 0):
+// What one CTA does with the partial sums of a row or momentum launch (enabled != 0): the last CTA of
+// that launch itself (FIN_LAST), where the host or the next launch needs the outcome at once
+// (stop_norm), or an extra CTA of the next tile launch (FIN_AHEAD), beside that launch's own work.
+// The reduction and the row's bookkeeping are a chain of dependent loads and sums, which at the end
+// of every step cost 2-4 us of a 13-60 us step.
 // kind 0: the observables row of step row_index (plus absorbed bookkeeping and stop_norm);
 // kind 1: the final observables (no bookkeeping); kind 2: only record the absorbed sums
 // of the next step's first accumAbsorbed.  [x0, x1): position-space and absorbed partial
@@ -318,19 +326,20 @@ struct NdFin {
     NdBook* book;
     // kind 0, renormalisation deferred (imaginary time): the launch summed the unnormalised psi.
     // The row is scaled as if psi had been normalised first (every sum by the factor squared, the
-    // autocorrelation by the factor), and the raw sum of |psi|^2 goes to *nsum_out, where the next
-    // step's first pass (TM_SCALE) or the final observables' pass (RM_SCALE) takes it from.
+    // autocorrelation by the factor), and the raw sum of |psi|^2 goes to *nsum_out, where the row pass
+    // that closes the next step, or the final observables' pass, takes it from (RM_SCALE).
     double* nsum_out;
     size_t x0, x1, k0, k1;
     double stop_norm;
     uint32_t mask;
     int row_index, kind, has_stop, enabled;
 };
+enum : int { FIN_LAST = 1, FIN_AHEAD = 2 };
 
 // true in the CTA that finishes last (its partials and everyone else's are visible to it)
 __device__ __forceinline__ bool nd_last_cta(unsigned* counter, unsigned total) {
     __shared__ bool last;
-    if (threadIdx.x < 32) __threadfence(); // the partial sums were written by the first warp
+    __threadfence(); // this thread's partial sums
     __syncthreads();
     if (threadIdx.x == 0) {
         last = atomicAdd(counter, 1u) == total - 1;
@@ -406,6 +415,12 @@ template <typename T> __device__ void nd_finalize_cta(const NdJob<T>& J, const N
         *F.rows_out = F.row_index + 1;
         if (F.has_stop && norm < F.stop_norm) *J.stopped = 1;
     }
+}
+
+// the sums of an earlier launch when no tile launch follows that could take them along
+template <typename T> __global__ void nd_finalize_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ NdFin F) {
+    if (*J.stopped) return;
+    nd_finalize_cta(J, F);
 }
 
 // index of grid point g along axis j (last axis fastest; n = 2^logn)
@@ -702,90 +717,138 @@ __device__ __forceinline__ void nd_observe(const NdJob<T>& J, const cx<T> (&x)[S
     }
 }
 
-// One sweep over the CTA's points (all S states of a point in one thread):
-// end of step i     1/N (after the inverse transform), accumAbsorbed + R, observables;
-//                   the values are copied to `phi_src` when given (momentum observables)
+// The stages of one grid point (all S states in one thread), after the inverse transform:
+// end of step i     1/N, accumAbsorbed + R, observables (x then holds the end-of-step state, copied
+//                   to `mid` when given: the momentum observables' input)
 // start of step i+1 accumAbsorbed + R
-// R is loaded once per point for both applications.  With one state a thread takes its
-// points in batches of four and loads the global inputs of the whole batch first (its
-// loads would otherwise wait one after the other); several states keep one point at a
-// time within the registers.  Returns after a barrier.
-// bx(line, x): where point x of line s L + l sits in buf (and phi_src).  OBSMAX: the observables
-// this instantiation can record (a compile-time bound on obs, so that a narrower form keeps fewer
-// accumulators and loads in registers).
-template <typename T, int D, int S, int NV, typename BX, uint32_t OBSMAX = ~0u>
-__device__ __forceinline__ void nd_row_sweep(const NdJob<T>& J, cx<T>* buf, cx<T>* phi_src, const BX& bx, int L, size_t row0,
-                                             uint32_t mode, uint32_t obs_in, double (&acc)[NV], bool wfn = true) {
+// R is loaded once for both applications.  obs: the observables to record, already bounded at
+// compile time by the caller where a narrower form drops the others' code and accumulators.  LEAN:
+// no absorbed-population tracking, wavefunction history or RM_NORM (their code compiled out).
+template <typename T, int D, int S, bool LEAN, int NV, typename A, typename MID>
+__device__ __forceinline__ void nd_row_point(const NdJob<T>& J, cx<T> (&v)[S], size_t g, uint32_t mode, uint32_t obs, const A& a,
+                                             T inv_n, double scale_f, bool wout, double (&acc)[NV], const MID& mid) {
     using SL = Slots<D, S>;
-    const uint32_t obs = obs_in & OBSMAX;
-    constexpr int SB = S == 1 ? 4 : 1;
-    using Aux = NdAux<T, S, (SB > 1)>;
-    const int logn = J.logn, pts = L << logn, nt = blockDim.x;
-    const T inv_n = (T)(1.0 / (double)J.N);
-    // RM_SCALE: the normalisation kernel's factors sqrt(dr * sum) and its square
-    const double nsq = (mode & RM_SCALE) ? sqrt(*J.nsum * J.dr) : 1.0, nden = nsq * nsq;
+    const bool adia = J.adiabatic && S > 1, track = !LEAN && J.track;
+    if (mode & RM_INV)
+#pragma unroll
+        for (int s = 0; s < S; ++s) v[s] = scale<T>(v[s], inv_n);
+    if (mode & RM_SCALE) // normalize (wavepacket.zig:282-284) with the norm of an earlier pass
+#pragma unroll
+        for (int s = 0; s < S; ++s) v[s] = nd_scaled<T>(v[s], scale_f);
+    if (mode & RM_REND) {
+        if (track) nd_absorbed<T, S, SL::abs>(J, v, g, a, acc);
+        a.R.apply(v);
+        if (!LEAN && (mode & RM_NORM))
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                acc[SL::norm] += (double)v[s].x * (double)v[s].x + (double)v[s].y * (double)v[s].y;
+    }
+    if (mode & RM_OBS) nd_observe<T, D, S>(J, v, g, obs, a, acc);
+    if (wout) { // History.append of the wavefunction (quantum_dynamics.zig:176-180), toAdia first (:919-927)
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            cx<T> y = v[i];
+            if (adia) {
+                double re = 0, im = 0;
+#pragma unroll
+                for (int k = 0; k < S; ++k) {
+                    const double u = a.u(J, g, k, i);
+                    re += (double)v[k].x * u;
+                    im += (double)v[k].y * u;
+                }
+                y = mk<T>((T)re, (T)im);
+            }
+            J.wfn_out[(size_t)i * J.N + g] = y;
+        }
+    }
+    mid(v);
+    if (mode & RM_RSTART) {
+        if (track) nd_absorbed<T, S, SL::absn>(J, v, g, a, acc);
+        a.R.apply(v);
+    }
+}
+
+// what the point stages of a row pass read besides psi
+template <typename T, int S, bool LEAN>
+__device__ __forceinline__ NdNeed nd_row_need(const NdJob<T>& J, uint32_t mode, uint32_t obs, bool wout) {
     const bool obsv = mode & RM_OBS, adia = J.adiabatic && S > 1;
     NdNeed nd;
     nd.R = mode & (RM_REND | RM_RSTART);
-    nd.w = J.track && nd.R;
-    const bool wout = wfn && J.wfn_out;
+    nd.w = !LEAN && J.track && nd.R;
     nd.U = adia && (nd.w || (obsv && (obs & WM_POP)) || wout);
     nd.V = obsv && (obs & (WM_EPOT | WM_ETOT));
     nd.z0 = obsv && (obs & WM_ACF);
+    return nd;
+}
+
+// One state: the stages of the sixteen points a thread holds (point t at g0 + t TPL), four at a time
+// with the global inputs of the four loaded first.  copy: where the end-of-step values go (element t
+// at copy[padf(t)], the thread's own elements), or null.
+template <typename T, int D, bool LEAN, int NV, int TPL, typename PF>
+__device__ __forceinline__ void nd_row_points(const NdJob<T>& J, cx<T> (&v)[16], size_t g0, uint32_t mode, uint32_t obs,
+                                              double (&acc)[NV], cx<T>* copy, const PF& padf) {
+    const T inv_n = (T)(1.0 / (double)J.N);
+    const double f = (mode & RM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
+    const bool wout = !LEAN && J.wfn_out != nullptr;
+    const NdNeed nd = nd_row_need<T, 1, LEAN>(J, mode, obs, wout);
+#pragma unroll
+    for (int t0 = 0; t0 < 16; t0 += 4) {
+        NdAux<T, 1, true> a[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) nd_aux_load<T, 1>(J, g0 + (t0 + b) * TPL, nd, a[b]);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            cx<T> x[1] = {v[t0 + b]};
+            nd_row_point<T, D, 1, LEAN>(J, x, g0 + (t0 + b) * TPL, mode, obs, a[b], inv_n, f, wout, acc, [&](const cx<T> (&y)[1]) {
+                if (copy) copy[padf(t0 + b)] = y[0];
+            });
+            v[t0 + b] = x[0];
+        }
+    }
+}
+
+// One sweep over the CTA's points (all S states of a point in one thread) in shared memory.
+// With one state a thread takes its points in batches of four and loads the global inputs of the
+// whole batch first (its loads would otherwise wait one after the other); several states keep one
+// point at a time within the registers, the next point's R (up to three states: six entries) loaded
+// ahead.  Returns after a barrier.  bx(line, x): where point x of line s L + l sits in buf (and phi_src).
+template <typename T, int D, int S, bool LEAN, int NV, typename BX>
+__device__ __forceinline__ void nd_row_sweep(const NdJob<T>& J, cx<T>* buf, cx<T>* phi_src, const BX& bx, int L, size_t row0,
+                                             uint32_t mode, uint32_t obs, double (&acc)[NV]) {
+    constexpr int SB = S == 1 ? 4 : 1;
+    constexpr bool AHEAD = S == 2 || S == 3;
+    using Aux = NdAux<T, S, (SB > 1)>;
+    const int logn = J.logn, pts = L << logn, nt = blockDim.x;
+    const T inv_n = (T)(1.0 / (double)J.N);
+    const double f = (mode & RM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
+    const bool wout = !LEAN && J.wfn_out != nullptr;
+    const NdNeed nd = nd_row_need<T, S, LEAN>(J, mode, obs, wout);
+    Aux nx;
+    if constexpr (AHEAD)
+        if ((int)threadIdx.x < pts) nd_aux_load<T, S>(J, row0 + threadIdx.x, nd, nx);
     for (int it0 = threadIdx.x; it0 < pts; it0 += SB * nt) {
         Aux a[SB];
+        if constexpr (AHEAD) {
+            a[0] = nx;
+            if (it0 + nt < pts) nd_aux_load<T, S>(J, row0 + it0 + nt, nd, nx);
+        } else {
 #pragma unroll
-        for (int b = 0; b < SB; ++b)
-            if (it0 + b * nt < pts) nd_aux_load<T, S>(J, row0 + it0 + b * nt, nd, a[b]);
+            for (int b = 0; b < SB; ++b)
+                if (it0 + b * nt < pts) nd_aux_load<T, S>(J, row0 + it0 + b * nt, nd, a[b]);
+        }
 #pragma unroll
         for (int b = 0; b < SB; ++b) {
             const int it = it0 + b * nt;
             if (it >= pts) break;
             const int l = it >> logn, x = it & ((1 << logn) - 1);
-            const size_t g = row0 + it;
             cx<T> v[S];
 #pragma unroll
             for (int s = 0; s < S; ++s) v[s] = buf[bx(s * L + l, x)];
-            if (mode & RM_INV)
+            nd_row_point<T, D, S, LEAN>(J, v, row0 + it, mode, obs, a[b], inv_n, f, wout, acc, [&](const cx<T> (&y)[S]) {
+                if (phi_src)
 #pragma unroll
-                for (int s = 0; s < S; ++s) v[s] = scale<T>(v[s], inv_n);
-            if (mode & RM_SCALE) // normalize (wavepacket.zig:282-284) with the norm of the previous pass
-#pragma unroll
-                for (int s = 0; s < S; ++s)
-                    v[s] = mk<T>((T)((double)v[s].x * nsq / nden), (T)((double)v[s].y * nsq / nden));
-            if (mode & RM_REND) {
-                if (J.track) nd_absorbed<T, S, SL::abs>(J, v, g, a[b], acc);
-                a[b].R.apply(v);
-                if (mode & RM_NORM)
-#pragma unroll
-                    for (int s = 0; s < S; ++s)
-                        acc[SL::norm] += (double)v[s].x * (double)v[s].x + (double)v[s].y * (double)v[s].y;
-            }
-            if (obsv) nd_observe<T, D, S>(J, v, g, obs, a[b], acc);
-            if (wout) { // History.append of the wavefunction (quantum_dynamics.zig:176-180), toAdia first (:919-927)
-#pragma unroll
-                for (int i = 0; i < S; ++i) {
-                    cx<T> y = v[i];
-                    if (adia) {
-                        double re = 0, im = 0;
-#pragma unroll
-                        for (int k = 0; k < S; ++k) {
-                            const double u = a[b].u(J, g, k, i);
-                            re += (double)v[k].x * u;
-                            im += (double)v[k].y * u;
-                        }
-                        y = mk<T>((T)re, (T)im);
-                    }
-                    J.wfn_out[(size_t)i * J.N + g] = y;
-                }
-            }
-            if (phi_src)
-#pragma unroll
-                for (int s = 0; s < S; ++s) phi_src[bx(s * L + l, x)] = v[s];
-            if (mode & RM_RSTART) {
-                if (J.track) nd_absorbed<T, S, SL::absn>(J, v, g, a[b], acc);
-                a[b].R.apply(v);
-            }
+                    for (int s = 0; s < S; ++s) phi_src[bx(s * L + l, x)] = y[s];
+            });
 #pragma unroll
             for (int s = 0; s < S; ++s) buf[bx(s * L + l, x)] = v[s];
         }
@@ -846,7 +909,7 @@ __global__ void __launch_bounds__(MAXT)
         double acc[SL::count];
 #pragma unroll
         for (int q = 0; q < SL::count; ++q) acc[q] = 0.0;
-        nd_row_sweep<T, D, S>(J, cur, (mode & RM_PHI) ? oth : nullptr,
+        nd_row_sweep<T, D, S, false, SL::count>(J, cur, (mode & RM_PHI) ? oth : (cx<T>*)nullptr,
                               [ldp](int line, int x) { return line * ldp + padx<T>(x); }, L, row0, mode, obs, acc);
         if (mode & (RM_OBS | RM_REND | RM_RSTART)) {
             // the slots this launch accumulates (nd_observe adds norm always, the rest by mask)
@@ -937,7 +1000,6 @@ __global__ void __launch_bounds__(512)
     const size_t outer = (size_t)blockIdx.x >> ltpo, inner0 = ((size_t)blockIdx.x & ((1u << ltpo) - 1)) << logt;
     const size_t c0 = ((outer << logn) << lstride) + inner0;
     cx<T>* data = ((mode & TM_PHI) ? J.phi : J.psi) + (size_t)blockIdx.y * J.N;
-    const double nf = (mode & TM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
     // element t of line g sits at data[c0 + (t << lstride) + g]; consecutive threads take consecutive lines
     cx<T> v[ND_IPT][8];
 #pragma unroll
@@ -948,9 +1010,6 @@ __global__ void __launch_bounds__(512)
             nd_item<true>(it, logt, logm, g, i);
 #pragma unroll
             for (int r = 0; r < 8; ++r) v[k][r] = data[c0 + ((size_t)(i + (r << logm)) << lstride) + g];
-            if (mode & TM_SCALE)
-#pragma unroll
-                for (int r = 0; r < 8; ++r) v[k][r] = nd_scaled<T>(v[k][r], nf);
         }
     }
     __syncthreads(); // twiddles staged
@@ -1031,18 +1090,37 @@ __global__ void __launch_bounds__(512)
     }
 }
 
-// ------------------------------------------------------------ tile pass, TMA-staged and persistent
-// A tile is W consecutive lines of one state along a strided axis, held as the TMA box lands:
-// element t of line g at t * W + g (rows of W * c bytes).  Each CTA loops over the tiles
-// k = blockIdx.x + j * gridDim.x; while it transforms tile j in one stage buffer, the TMA load
-// of tile j + 1 fills the other, and tile j leaves through a TMA store.  The radix passes run in
-// place in the stage buffer (every thread reads its inputs, a barrier, then the writes), so a
-// tile needs no second line buffer; the first and last radix-8 passes stay in registers.
-// TM_KOBS (the momentum observables of phi after its forward transform along axis 0) stores
-// nothing: its sums run over the CTA's tiles and are written once, at column blockIdx.x.
-constexpr int NDT_STAGES = 2;
+// ------------------------------------------------------------ TMA-staged persistent passes
+// Both passes keep sixteen elements of a line per thread in registers (nd_fft.cuh).  A CTA loops
+// over its items k = blockIdx.x + j * workers; an item's elements arrive in a shared-memory stage by
+// TMA, go to registers, through the transforms (whose pass boundaries use the exchange buffer) and
+// from registers straight back to global memory.  Where the shape has room the exchange buffer is
+// separate from the stage, and the next item's load is issued as soon as every thread has read the
+// stage; otherwise the two share their space and the next load is issued when the item is done
+// (several CTAs per SM then overlap one another's loads).  Lines of at most 512 points belong to
+// one warp each, so their transforms wait at no CTA barrier.
 constexpr long long NDT_WAIT_CYCLES = 4000000000LL; // ~2 s: a TMA load that has not landed by then has failed
 // (the default budget of the waits; a test of the failure path passes a short one)
+
+// shared memory of a TMA-staged pass of nl lines of n points: the stage, the exchange buffer (the
+// same space when shared), the row pass's copy of the end-of-step lines (momentum copies only), the
+// twiddles, the mbarriers, and slack to align the whole
+struct NdtSmem {
+    size_t stage, exch, copy, tw, bars, total;
+};
+template <typename T>
+__host__ __device__ inline NdtSmem ndt_smem(int nl, int n, int ldx, bool shared, bool copy) {
+    auto up = [](size_t b) { return (b + 127) & ~(size_t)127; };
+    const size_t st = up((size_t)nl * n * sizeof(cx<T>)), ex = up((size_t)nl * ldx * sizeof(cx<T>));
+    NdtSmem m;
+    m.stage = 0;
+    m.exch = shared ? 0 : st;
+    m.copy = shared ? (ex > st ? ex : st) : st + ex;
+    m.tw = m.copy + (copy ? ex : 0);
+    m.bars = m.tw + (size_t)n * sizeof(Tab<T>);
+    m.total = m.bars + 2 * sizeof(uint64_t) + 128;
+    return m;
+}
 
 struct NdTma {
     int axis;
@@ -1051,133 +1129,76 @@ struct NdTma {
     int logtiles;   // tiles per state
     int logO;       // outer lines (planes of the tensor map) per state
     unsigned nitems; // tiles of all states
-    unsigned ncols;  // TM_KOBS: columns of the partial-sum region (written whole)
+    unsigned workers; // CTAs that take items
+    int shared;      // the stage and the exchange buffer share their space
+    int ldx;         // exchange line stride
     long long wait_cycles; // budget of each mbarrier wait
     int withhold;    // testing: each CTA's first load is not issued, so its wait runs out
 };
 
-template <typename T> __host__ __device__ inline size_t ndt_stage_bytes(int W, int n) { return (size_t)W * n * sizeof(cx<T>); }
-// stages, twiddles (W_n, then both directions' middle-pass tables), the stage mbarriers, and
-// 128 bytes of slack to align the stages
-template <typename T> __host__ __device__ inline size_t ndt_smem_bytes(int W, int n) {
-    return 128 + (size_t)NDT_STAGES * ndt_stage_bytes<T>(W, n) + (size_t)(n + 2 * nd_mid_tw(n)) * sizeof(Tab<T>) +
-           NDT_STAGES * sizeof(uint64_t);
-}
-
-// Where element t of line g of a stage sits, and which (line, butterfly) pair item `it` of a
-// pass handles.  IxTile: the strided-axis tile, t-major as the TMA box lands (t W + g), lines
-// fastest across threads.  IxRow: lines of the last axis, line-major (g n + t) under the 128-byte
-// TMA swizzle (16-byte chunk j of 128-byte row q stored at chunk j ^ (q mod 8)), points fastest.
-struct IxTile {
-    int logW;
-    __device__ __forceinline__ int at(int g, int t) const { return (t << logW) + g; }
-    __device__ __forceinline__ void item(int it, int logi, int& g, int& i) const {
-        g = it & ((1 << logW) - 1);
-        i = it >> logW;
-        (void)logi;
+// The CTA's sums of the values set in `act` (uniform) over all its threads, compensated, to column
+// `col` of slots first .. first + NV of part (the others as zero).  red: shared memory for eight
+// doubles a thread, free to use; whole warps.  Each value is summed by one warp from the threads'
+// sums laid side by side: a shuffle tree per warp and value cost an eighth of a short pass.
+template <int NV>
+__device__ __forceinline__ void cta_partials(const double (&a)[NV], uint32_t act, double* __restrict__ red, int first,
+                                             double* __restrict__ part, size_t P, size_t col) {
+    const int nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, nw = nt >> 5;
+    const int nact = __popc(act);
+    if (tid < NV && !((act >> tid) & 1u)) {
+        const size_t o = ((size_t)(first + tid) * P + col) * 2;
+        part[o] = 0.0;
+        part[o + 1] = 0.0;
     }
-};
-template <typename T> struct IxRow {
-    int logn;
-    __device__ __forceinline__ int operator()(int g, int t) const { return at(g, t); }
-    __device__ __forceinline__ int at(int g, int t) const {
-        const int e = (g << logn) + t;
-        if constexpr (sizeof(cx<T>) == 16) return e ^ ((e >> 3) & 7);
-        else return e ^ (((e >> 4) & 7) << 1);
-    }
-    __device__ __forceinline__ void item(int it, int logi, int& g, int& i) const {
-        i = it & ((1 << logi) - 1);
-        g = it >> logi;
-    }
-};
-
-// In-place radix-R Stockham pass over a stage's lines.  Butterfly (g, i), i < n/R, reads
-// elements i + r n/R and writes o0 + r p; all reads come before the barrier, all writes after
-// it.  twp: W_n^(r kk n/(p R)) at [(r - 1) p + kk].
-template <typename T, int R, int SIGN, typename IX>
-__device__ __forceinline__ void ndt_pass(cx<T>* buf, const IX& ix, int logn, int p, const Tab<T>* __restrict__ twp) {
-    constexpr int LR = R == 2 ? 1 : R == 4 ? 2 : 3;
-    constexpr int B = 8 / R; // butterflies per thread (the CTA has one thread per 8 points)
-    const int logmr = logn - LR, nt = blockDim.x;
-    cx<T> v[B][R];
+    for (int c0 = 0; c0 < nact; c0 += 8) {
+        __syncthreads();
 #pragma unroll
-    for (int b = 0; b < B; ++b) {
-        int g, i;
-        ix.item(threadIdx.x + b * nt, logmr, g, i);
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[b][r] = buf[ix.at(g, i + (r << logmr))];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-        int g, i;
-        ix.item(threadIdx.x + b * nt, logmr, g, i);
-        const int kk = i & (p - 1);
-        if (p > 1) {
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[b][r] = tmul<SIGN>(v[b][r], twp[(r - 1) * p + kk]);
+        for (int v = 0; v < NV; ++v) {
+            const int k = __popc(act & ((1u << v) - 1u)) - c0;
+            if (((act >> v) & 1u) && k >= 0 && k < 8) red[k * nt + tid] = a[v];
         }
-        dft<R, SIGN, T>(v[b]);
-        const int o0 = ((i - kk) << LR) + kk;
+        __syncthreads();
+        for (int k = tid >> 5; k < 8 && c0 + k < nact; k += nw) {
+            Acc t;
+            for (int e = lane; e < nt; e += 32) t.add(red[k * nt + e]);
 #pragma unroll
-        for (int r = 0; r < R; ++r) buf[ix.at(g, o0 + r * p)] = v[b][r];
-    }
-    __syncthreads();
-}
-
-// One n-point transform of a stage's lines, in place.  In: v[r] = element i + r n/8 of line g
-// (the thread's item).  Out: the same elements of the transformed line.  The buffer's contents
-// are free on entry (the barrier before the first write lets every thread finish reading it)
-// and hold nothing of value on return.
-template <typename T, int SIGN, typename IX>
-__device__ __forceinline__ void ndt_fft(cx<T> (&v)[8], cx<T>* buf, const IX& ix, int logn, const Tab<T>* __restrict__ twm) {
-    dft<8, SIGN, T>(v);
-    if (logn == 3) return;
-    const NdSched sc = nd_sched(logn);
-    const int logm = logn - 3;
-    int g, i;
-    ix.item(threadIdx.x, logm, g, i);
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 8; ++r) buf[ix.at(g, (i << 3) + r)] = v[r]; // first pass, p = 1: outputs at 8 i + r
-    __syncthreads();
-    const Tab<T>* twd = twm + (1 << logn) + (SIGN > 0 ? nd_mid_tw(1 << logn) : 0);
-    int logp = 3, tbase = 0;
-    for (int j = 0; j < sc.nmid; ++j) {
-        const int lr = sc.lr(j, SIGN > 0 && sc.last8), p = 1 << logp;
-        if (lr == 3) ndt_pass<T, 8, SIGN>(buf, ix, logn, p, twd + tbase);
-        else if (lr == 2) ndt_pass<T, 4, SIGN>(buf, ix, logn, p, twd + tbase);
-        else ndt_pass<T, 2, SIGN>(buf, ix, logn, p, twd + tbase);
-        tbase += ((1 << lr) - 1) * p;
-        logp += lr;
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = buf[ix.at(g, i + (r << logm))];
-    if (sc.last8) { // last radix-8 pass, p = n/8: twiddle W_n^(r i)
-#pragma unroll
-        for (int r = 1; r < 8; ++r) v[r] = tmul<SIGN>(v[r], twm[r * i]);
-        dft<8, SIGN, T>(v);
+            for (int off = 16; off > 0; off >>= 1) {
+                const double s2 = __shfl_down_sync(0xffffffffu, t.s, off), c2 = __shfl_down_sync(0xffffffffu, t.c, off);
+                t.add(s2);
+                t.c += c2;
+            }
+            if (lane == 0) {
+                const int v = __fns(act, 0, c0 + k + 1);
+                const size_t o = ((size_t)(first + v) * P + col) * 2;
+                part[o] = t.s;
+                part[o + 1] = t.c;
+            }
+        }
     }
 }
 
 // map: 3-D tensor map of this axis over psi in 8-byte words: [E * stride] words (the inner
-// lines), [n] rows along the axis, [S * O] planes (outer index and state); box [E W, min(n, 256), 1]
-template <typename T, int D>
-__global__ void __launch_bounds__(512)
+// lines), [n] rows along the axis, [S * O] planes (outer index and state); box [E W, min(n, 256), 1].
+// The stage holds element t of line g at t W + g, as the box lands.
+// TM_KOBS (the momentum observables of phi after its forward transform along axis 0) stores
+// nothing: its sums run over the CTA's tiles and are written once, at column blockIdx.x.
+template <typename T, int D, int LOGN>
+__global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     nd_tile_tma_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ CUtensorMap map, const NdTma P,
                        size_t part_base, const __grid_constant__ NdFin F) {
-    if (*J.stopped) return;
+    using PL = LinePlan<LOGN>;
+    constexpr int n = PL::n, TPL = PL::TPL, E = (int)(sizeof(cx<T>) / 8);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-    const int n = J.n, logn = J.logn, logm = logn - 3, logW = P.logW, W = 1 << logW;
-    const int lstride = logn * (D - 1 - P.axis);
-    constexpr int E = (int)(sizeof(cx<T>) / 8);
-    const size_t sb = ndt_stage_bytes<T>(W, n);
-    cx<T>* stage0 = reinterpret_cast<cx<T>*>(base);
-    Tab<T>* twm = reinterpret_cast<Tab<T>*>(base + NDT_STAGES * sb);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(twm + n + 2 * nd_mid_tw(n));
-    const int tid = threadIdx.x, g = tid & (W - 1), i = tid >> logW;
-    const int rows = n < 256 ? n : 256;
+    const int logW = P.logW, W = 1 << logW, tid = threadIdx.x;
+    const NdtSmem M = ndt_smem<T>(W, n, P.ldx, P.shared, false);
+    cx<T>* stage = reinterpret_cast<cx<T>*>(base + M.stage);
+    cx<T>* exch = reinterpret_cast<cx<T>*>(base + M.exch);
+    Tab<T>* tw = reinterpret_cast<Tab<T>*>(base + M.tw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + M.bars);
+    const int lstride = LOGN * (D - 1 - P.axis);
+    const unsigned sb = (unsigned)((size_t)W * n * sizeof(cx<T>));
+    constexpr int rows = n < 256 ? n : 256;
     // tile k: state s = k >> logtiles, lines l0 = (k mod tiles) W of that state; box origin
     // x = E (l0 mod stride) words, plane z = s O + l0 / stride
     auto origin = [&](unsigned k, int& x, int& z, size_t& gbase) {
@@ -1186,210 +1207,200 @@ __global__ void __launch_bounds__(512)
         const size_t inner0 = l0 & (((size_t)1 << lstride) - 1), outer = l0 >> lstride;
         x = E * (int)inner0;
         z = (int)(((size_t)s << P.logO) + outer);
-        gbase = ((outer << logn) << lstride) + inner0; // grid index of element 0 of the tile's line 0
+        gbase = ((outer << LOGN) << lstride) + inner0; // grid index of element 0 of the tile's line 0
     };
-    auto issue = [&](unsigned k, int st) {
+    auto issue = [&](unsigned k) {
         int x, z;
         size_t gb;
         origin(k, x, z, gb);
-        cx<T>* dst = stage0 + (size_t)st * W * n;
-        mbar_arrive_expect_tx(&bars[st], (unsigned)sb);
-        for (int y = 0; y < n; y += rows) tma_load_3d(dst + (size_t)y * W, &map, x, y, z, &bars[st]);
+        mbar_arrive_expect_tx(&bars[0], sb);
+        for (int y = 0; y < n; y += rows) tma_load_3d(stage + (size_t)y * W, &map, x, y, z, &bars[0]);
     };
     if (tid == 0) {
         prefetch_tensormap(&map);
-#pragma unroll
-        for (int s = 0; s < NDT_STAGES; ++s) mbar_init(&bars[s], 1);
+        mbar_init(&bars[0], 1);
         fence_barrier_init();
-        // the first load overlaps the twiddle staging (the stages and the twiddles do not overlap)
-        if (blockIdx.x < P.nitems && !P.withhold) issue(blockIdx.x, 0);
     }
-    for (int t = tid; t < n; t += blockDim.x) twm[t] = J.tw[t];
-    nd_stage_mid_tw<T>(J.tw, twm + n, logn);
+    const int stopped = *J.stopped; // read beside the first load, not before it
+    if (blockIdx.x >= P.workers) {  // the extra CTA: an earlier launch's sums
+        if (!stopped) nd_finalize_cta(J, F);
+        return;
+    }
+    // the first load overlaps the twiddle staging (the stage and the twiddles do not overlap)
+    if (tid == 0 && !P.withhold) issue(blockIdx.x);
+    for (int t = tid; t < PL::ntw; t += blockDim.x) tw[t] = J.twd[t];
     __syncthreads();
+    // the thread's line g of the tile and its place i in the line: a warp takes whole lines where
+    // they are short enough, neighbouring threads neighbouring lines
+    constexpr bool WARP = TPL <= 32;
+    constexpr int LPW = WARP ? 32 / TPL : 1;
+    const int g = WARP ? (tid >> 5) * LPW + (tid & (LPW - 1)) : tid & (W - 1);
+    const int i = WARP ? (tid & 31) / LPW : tid >> logW;
+    using SY = typename std::conditional<WARP, SyncWarp, SyncCta>::type;
+    const SY sync{};
+    cx<T>* line = exch + (size_t)g * P.ldx;
     const bool kobs = P.mode & TM_KOBS;
-    const double nf = (P.mode & TM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
     double acc[D + 1]; // TM_KOBS: <k_j> sums and the kinetic energy's, over the CTA's tiles
 #pragma unroll
     for (int a = 0; a <= D; ++a) acc[a] = 0.0;
     bool failed = false;
-    int j = 0;
-    for (unsigned k = blockIdx.x; k < P.nitems; k += gridDim.x, ++j) {
-        const int st = j & 1;
-        const unsigned kn = k + gridDim.x;
-        if (j > 0 && kobs) __syncthreads(); // every thread is done with tile j - 1's stage (not stored)
-        if (tid == 0 && kn < P.nitems) {
-            bulk_wait_read_all(); // the store of tile j - 1 has read the other stage
-            issue(kn, st ^ 1);
-        }
-        const bool ok = mbar_wait_bounded(&bars[st], (unsigned)(j >> 1) & 1u, P.wait_cycles);
-        if (!__syncthreads_and(ok)) { // the load never landed: record it, let the prefetch land, stop
-            if (tid == 0) {
-                atomicExch(J.err, 1);
-                if (kn < P.nitems) mbar_wait_bounded(&bars[st ^ 1], (unsigned)((j + 1) >> 1) & 1u, P.wait_cycles);
-            }
-            failed = true;
-            break;
-        }
-        cx<T>* buf = stage0 + (size_t)st * W * n;
+    unsigned j = 0;
+    for (unsigned k = blockIdx.x; k < P.nitems; k += P.workers, ++j) {
+        const unsigned kn = k + P.workers;
+        const bool ok = mbar_wait_bounded(&bars[0], j & 1u, P.wait_cycles);
+        if (stopped) return; // the first load has landed (or the wait ran out) and none other is in flight
         int x, z;
         size_t gbase;
         origin(k, x, z, gbase);
-        const IxTile ix{logW};
-        cx<T> v[8];
+        cx<T> v[16];
+        if (ok) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = buf[ix.at(g, i + (r << logm))];
-        if (P.mode & TM_SCALE)
-#pragma unroll
-            for (int r = 0; r < 8; ++r) v[r] = nd_scaled<T>(v[r], nf);
-        if (P.mode & TM_FWD) ndt_fft<T, -1>(v, buf, ix, logn, twm);
+            for (int t = 0; t < 16; ++t) v[t] = stage[((i + t * TPL) << logW) + g];
+        }
+        if (!P.shared) fence_async_smem(); // this thread's reads of the stage, before the next load's writes
+        if (!__syncthreads_and(ok)) { // the load never landed: record it and stop (none is in flight after it)
+            if (tid == 0) atomicExch(J.err, 1);
+            failed = true;
+            break;
+        }
+        if (tid == 0 && !P.shared && kn < P.nitems) issue(kn); // every thread has read the stage
+        if (P.mode & TM_FWD) line_fft<T, LOGN, -1>(v, line, i, tw, sync);
+        const size_t gl = gbase + g;
         if (P.mode & TM_KPHASE) {
             // exp(Complex(0, -K) * dt), K = sum_j k_j^2 / (2 m_j) (quantum_dynamics.zig:397-399), as the
             // product of per-axis factors: the line's other axes once, then one product per element
-            const size_t gl = gbase + g;
             double2 fl = make_double2(1.0, 0.0);
 #pragma unroll
             for (int a = 0; a < D; ++a)
-                if (a != P.axis) {
-                    const double2 e = J.kphase[a * n + axis_index<D>(gl, a, logn)];
-                    fl = make_double2(__dsub_rn(__dmul_rn(fl.x, e.x), __dmul_rn(fl.y, e.y)),
-                                      __dadd_rn(__dmul_rn(fl.x, e.y), __dmul_rn(fl.y, e.x)));
-                }
+                if (a != P.axis) fl = mul<double>(fl, J.kphase[a * n + axis_index<D>(gl, a, LOGN)]);
+            const double2* __restrict__ f0 = J.kphase + P.axis * n + i;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const double2 f0 = J.kphase[P.axis * n + i + (r << logm)];
-                const double2 f = make_double2(__dsub_rn(__dmul_rn(f0.x, fl.x), __dmul_rn(f0.y, fl.y)),
-                                               __dadd_rn(__dmul_rn(f0.x, fl.y), __dmul_rn(f0.y, fl.x)));
-                v[r] = tmul<-1>(v[r], mktab<T>(f.x, f.y));
+            for (int t = 0; t < 16; ++t) {
+                const double2 f = mul<double>(f0[t * TPL], fl);
+                v[t] = tmul<-1>(v[t], mktab<T>(f.x, f.y));
             }
         }
         if (kobs) { // Wavefunction.mom / ekin (wavepacket.zig:224-232, 258-268), per-axis tables
-            const size_t gl = gbase + g;
             double Kl = 0, kl[D];
 #pragma unroll
             for (int a = 0; a < D; ++a) {
                 kl[a] = 0;
                 if (a != P.axis) {
-                    const double4 e = J.axis[a * n + axis_index<D>(gl, a, logn)];
+                    const double4 e = J.axis[a * n + axis_index<D>(gl, a, LOGN)];
                     Kl += e.z;
                     kl[a] = e.y;
                 }
             }
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const double4 a0 = J.axis[P.axis * n + i + (r << logm)];
-                const double w = (double)v[r].x * (double)v[r].x + (double)v[r].y * (double)v[r].y;
+            for (int t = 0; t < 16; ++t) {
+                const double4 a0 = J.axis[P.axis * n + i + t * TPL];
+                const double w = (double)v[t].x * (double)v[t].x + (double)v[t].y * (double)v[t].y;
 #pragma unroll
                 for (int a = 0; a < D; ++a) acc[a] += w * (a == P.axis ? a0.y : kl[a]);
                 acc[D] += w * (Kl + a0.z);
             }
-            continue; // no store
-        }
-        if (P.mode & TM_INV) ndt_fft<T, 1>(v, buf, ix, logn, twm);
-        __syncthreads(); // every thread's last-pass reads are done
+        } else {
+            if (P.mode & TM_INV) {
+                if (P.mode & TM_FWD) sync(); // the line's last exchange has been read
+                line_fft<T, LOGN, 1>(v, line, i, tw, sync);
+            }
+            cx<T>* dst = ((P.mode & TM_PHI) ? J.phi : J.psi) + ((size_t)(k >> P.logtiles)) * J.N + gl + ((size_t)i << lstride);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) buf[ix.at(g, i + (r << logm))] = v[r];
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            for (int y = 0; y < n; y += rows) tma_store_3d(&map, x, y, z, buf + (size_t)y * W);
-            bulk_commit();
+            for (int t = 0; t < 16; ++t) dst[(size_t)(t * TPL) << lstride] = v[t];
+        }
+        if (P.shared) {
+            fence_async_smem(); // the exchange's writes, before the next load's
+            __syncthreads();
+            if (tid == 0 && kn < P.nitems) issue(kn);
+        } else {
+            sync(); // the line's last exchange has been read before the next item writes it
         }
     }
-    if (tid == 0) bulk_wait_all();
     if (!kobs || failed) return;
-    block_partials<D + 1>(acc, Slots<D, 1>::mom, J.part, J.nparts, part_base + blockIdx.x);
-    for (size_t col = blockIdx.x + gridDim.x; col < P.ncols; col += gridDim.x) // columns no CTA owns
-        for (int a = tid; a <= D; a += blockDim.x) {
-            const size_t o = ((size_t)(Slots<D, 1>::mom + a) * J.nparts + part_base + col) * 2;
-            J.part[o] = 0.0;
-            J.part[o + 1] = 0.0;
-        }
-    if (F.enabled && nd_last_cta(&F.book->counter, gridDim.x)) nd_finalize_cta(J, F);
+    __syncthreads();
+    cta_partials<D + 1>(acc, (1u << (D + 1)) - 1u, reinterpret_cast<double*>(exch), Slots<D, 1>::mom, J.part, J.nparts,
+                        part_base + blockIdx.x);
+    if (F.enabled == FIN_LAST && nd_last_cta(&F.book->counter, P.workers)) nd_finalize_cta(J, F);
 }
 
 // ------------------------------------------------------------ row pass, TMA-staged and persistent
 // An item is a block of L rows of the last axis with all S states (the row pass's unit of work);
-// its stage holds line g = s L + l (g n + t, 128-byte swizzled, IxRow) as the TMA boxes land.
-// Each CTA loops over the blocks k = blockIdx.x + j * gridDim.x with the next block's load in
-// flight and the next block's propagator table prefetched into L2.  The observables' sums run
-// over all of a CTA's blocks and are written once, at column blockIdx.x of the partial array
-// (the grid's size is fixed per job and device); the columns no CTA owns are written as zero so
-// that the region stays whole.  Modes: any
-// combination of the row-pass modes.  RM_PHI keeps the end-of-step state in registers while the
-// start of the next step is applied, and transforms it through the stage after the psi store has
-// read it; it leaves through map_phi.
+// its stage holds line g = s L + l at g n.  The per-point stages between the two transforms run on
+// the registers of the line's threads for one state; several states meet in one thread through the
+// exchange buffer (nd_row_sweep).  The observables' sums run over all of a CTA's blocks and are
+// written once, at column blockIdx.x of the partial array (the grid's size is fixed per job and
+// device).  Modes: any combination of the row-pass modes.  RM_PHI keeps a copy of the end-of-step
+// state beside the exchange buffer and transforms it into phi.
 struct NdRowTma {
     uint32_t mode, obs;
     int logL;        // rows per block
-    unsigned nitems; // blocks, and columns of the partial-sum region
+    unsigned nitems; // blocks
+    unsigned workers; // CTAs that take blocks
+    unsigned ncols;   // columns of the partial-sum region (written whole)
+    int shared;      // the stage and the exchange buffer share their space
+    int ldx;         // exchange line stride
     long long wait_cycles; // budget of each mbarrier wait
     int withhold;    // testing: each CTA's first load is not issued, so its wait runs out
 };
-
-template <typename T> __host__ __device__ inline size_t ndr_stage_bytes(int S, int L, int n) {
-    return (size_t)S * L * n * sizeof(cx<T>);
-}
-// 1024 bytes of slack to align the stages (the 128-byte swizzle repeats every 1024 bytes), the
-// stages, the twiddles, the stage mbarriers
-template <typename T> __host__ __device__ inline size_t ndr_smem_bytes(int S, int L, int n) {
-    return 1024 + (size_t)NDT_STAGES * ndr_stage_bytes<T>(S, L, n) + (size_t)(n + 2 * nd_mid_tw(n)) * sizeof(Tab<T>) +
-           NDT_STAGES * sizeof(uint64_t);
-}
 
 __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(p)), "r"(bytes) : "memory");
 }
 
-// map: 3-D tensor map over psi as rows of 128 bytes: [16 words] x [S N c / 128 rows] x [1],
-// box [16, min(256, L n c / 128), 1], 128-byte swizzle
-// The TMA row pass's CTA size bound MAXT: 256 threads, two CTAs per SM (128 registers) for the
-// plain forms, one for the form with the momentum copy (its registers hold the end-of-step state
-// as well); 512 threads, one CTA per SM (128 registers), for the plain forms of one or two
-// states on long lines.
-constexpr int NDR_THREADS = 256, NDR_THREADS_WIDE = 512;
+constexpr int NDR_THREADS = 256;
 
-// POP: the form for steps that record only the populations and the norm (the other observables'
-// code and accumulators compiled out), three CTAs per SM (80 registers) for one or two states.
-template <typename T, int D, int S, bool PHI, int MAXT = NDR_THREADS, bool POP = false>
-__global__ void __launch_bounds__(MAXT, MAXT == NDR_THREADS && !PHI ? (POP && S <= 2 ? 3 : 2) : 1)
-    nd_row_tma_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ CUtensorMap map,
-                      const __grid_constant__ CUtensorMap map_phi, const NdRowTma P, size_t part_base,
+// The forms of the row kernel: which observables its code can record, and whether it is lean
+// (nd_row_point).  What a launch does not record costs registers all the same unless it is compiled
+// out: with everything in one form the FP64 kernels spilled one to two kilobytes a thread.
+enum : int { RF_GENERAL = 0, RF_POP = 1, RF_ACF = 2, RF_ALL = 3, RF_COUNT = 4 };
+constexpr uint32_t row_form_obs(int form) {
+    return form == RF_POP ? (uint32_t)(WM_POP | WM_NORM) : form == RF_ACF ? (uint32_t)(WM_ACF | WM_NORM) : ~0u;
+}
+// The row kernel's registers a thread, as the thread count whose one CTA would fill the register file
+// (512: 128 registers, 384: 168, 416: 152, 608: 104; CTAs have at most 256 threads).  FP64 holds 64 of
+// data (one state's sixteen points); the per-point stages of several states want more than 128, which
+// CTAs of at most 192 threads have room for and the 256-thread CTAs of the longest lines do not (two
+// of them share an SM: 2048^2 x 2 states FP64 294 -> 256 us a step, while 1024^2 x 3 would lose, 102 -> 114).
+template <typename T> constexpr int row_bound(int S, int logn, int form) {
+    const bool narrow = S == 1 && (form == RF_POP || form == RF_ACF);
+    if (S >= 2 && logn >= 11) return 512;
+    return sizeof(T) == 8 ? (narrow ? 512 : 384) : narrow ? 608 : S <= 2 ? 512 : 416;
+}
+
+template <typename T, int D, int S, int LOGN, int FORM>
+__global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
+    nd_row_tma_kernel(const __grid_constant__ NdJob<T> J, const NdRowTma P, size_t part_base,
                       const __grid_constant__ NdFin F) {
-    if (*J.stopped) return;
     using SL = Slots<D, S>;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int n = J.n, logn = J.logn, logm = logn - 3, L = 1 << P.logL;
-    const size_t sb = ndr_stage_bytes<T>(S, L, n), blk = (size_t)L * n; // points of one state in a block
-    cx<T>* stage0 = reinterpret_cast<cx<T>*>(base);
-    Tab<T>* twm = reinterpret_cast<Tab<T>*>(base + NDT_STAGES * sb);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(twm + n + 2 * nd_mid_tw(n));
-    const int tid = threadIdx.x;
-    const unsigned rows_state = (unsigned)(blk * sizeof(cx<T>) / 128), rows_box = rows_state < 256 ? rows_state : 256;
-    const uint32_t mode = PHI ? P.mode : (P.mode & ~(uint32_t)RM_PHI);
+    using PL = LinePlan<LOGN>;
+    constexpr int n = PL::n, TPL = PL::TPL;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    const int L = 1 << P.logL, tid = threadIdx.x;
+    const uint32_t mode = P.mode;
+    const NdtSmem M = ndt_smem<T>(S * L, n, P.ldx, P.shared, mode & RM_PHI);
+    cx<T>* stage = reinterpret_cast<cx<T>*>(base + M.stage);
+    cx<T>* exch = reinterpret_cast<cx<T>*>(base + M.exch);
+    cx<T>* copy = reinterpret_cast<cx<T>*>(base + M.copy);
+    Tab<T>* tw = reinterpret_cast<Tab<T>*>(base + M.tw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + M.bars);
+    const size_t blk = (size_t)L << LOGN; // points of one state in a block
+    const unsigned sb = (unsigned)(blk * sizeof(cx<T>));
     const bool needR = mode & (RM_REND | RM_RSTART);
-    auto issue = [&](unsigned k, int st) {
-        unsigned char* dst = base + (size_t)st * sb;
-        mbar_arrive_expect_tx(&bars[st], (unsigned)sb);
-        for (int s = 0; s < S; ++s) {
-            const size_t row = ((size_t)s * J.N + (size_t)k * blk) * sizeof(cx<T>) / 128;
-            for (unsigned y = 0; y < rows_state; y += rows_box)
-                tma_load_3d(dst + ((size_t)s * rows_state + y) * 128, &map, 0, (int)(row + y), 0, &bars[st]);
-        }
+    auto issue = [&](unsigned k) {
+        mbar_arrive_expect_tx(&bars[0], S * sb);
+        for (int s = 0; s < S; ++s) bulk_load(stage + (size_t)s * blk, J.psi + (size_t)s * J.N + (size_t)k * blk, sb, &bars[0]);
         if (needR) // the block's propagator entries, for the sweep's loads
             for (int c = 0; c < S * (S + 1) / 2; ++c) prefetch_l2(J.R + (size_t)c * J.N + (size_t)k * blk, (unsigned)(blk * sizeof(Tab<T>)));
     };
     if (tid == 0) {
-        prefetch_tensormap(&map);
-#pragma unroll
-        for (int s = 0; s < NDT_STAGES; ++s) mbar_init(&bars[s], 1);
+        mbar_init(&bars[0], 1);
         fence_barrier_init();
-        // the first load overlaps the twiddle staging (the stages and the twiddles do not overlap)
-        if (blockIdx.x < P.nitems && !P.withhold) issue(blockIdx.x, 0);
     }
-    for (int t = tid; t < n; t += blockDim.x) twm[t] = J.tw[t];
-    nd_stage_mid_tw<T>(J.tw, twm + n, logn);
+    const int stopped = *J.stopped; // read beside the first load, not before it
+    // the first load overlaps the twiddle staging (the stage and the twiddles do not overlap)
+    if (tid == 0 && !P.withhold) issue(blockIdx.x);
+    for (int t = tid; t < PL::ntw; t += blockDim.x) tw[t] = J.twd[t];
     __syncthreads();
     const bool sums = mode & (RM_OBS | RM_REND | RM_RSTART);
     uint32_t act = 1u << SL::norm; // the slots this launch accumulates (nd_observe adds norm always)
@@ -1401,111 +1412,108 @@ __global__ void __launch_bounds__(MAXT, MAXT == NDR_THREADS && !PHI ? (POP && S 
             if (P.obs & WM_ACF) act |= 3u << SL::acf;
             if (P.obs & WM_POP) act |= sm << SL::pop;
         }
-        if (J.track) act |= (sm << SL::abs) | (sm << SL::absn);
+        if (FORM == RF_GENERAL && J.track) act |= (sm << SL::abs) | (sm << SL::absn);
     }
+    constexpr bool LEAN = FORM != RF_GENERAL;
+    const uint32_t obs = P.obs & row_form_obs(FORM);
     double acc[SL::count];
 #pragma unroll
     for (int q = 0; q < SL::count; ++q) acc[q] = 0.0;
-    const IxRow<T> ix{logn};
-    int g, i;
-    ix.item(tid, logm, g, i);
+    const int g = tid / TPL, i = tid & (TPL - 1); // the thread's line and its place in it
+    const int gs = S == 1 ? 0 : g / L;            // the line's state
+    using SY = typename std::conditional<TPL <= 32, SyncWarp, SyncBar>::type;
+    SY sync;
+    if constexpr (TPL > 32) {
+        sync.id = 1 + g;
+        sync.count = TPL;
+    }
+    cx<T>* line = exch + (size_t)g * P.ldx;
+    cx<T>* cline = copy + (size_t)g * P.ldx;
     bool failed = false;
-    int j = 0;
-    for (unsigned k = blockIdx.x; k < P.nitems; k += gridDim.x, ++j) {
-        const int st = j & 1;
-        const unsigned kn = k + gridDim.x;
-        if (j > 0) __syncthreads(); // every thread is done with block j - 1's stage (a block need not be stored)
-        if (tid == 0 && kn < P.nitems) {
-            bulk_wait_read_all(); // the store of block j - 1 has read the other stage
-            issue(kn, st ^ 1);
+    unsigned j = 0;
+    for (unsigned k = blockIdx.x; k < P.nitems; k += P.workers, ++j) {
+        const unsigned kn = k + P.workers;
+        const bool ok = mbar_wait_bounded(&bars[0], j & 1u, P.wait_cycles);
+        if (stopped) return; // the first load has landed (or the wait ran out) and none other is in flight
+        cx<T> v[16];
+        if (ok) {
+            const cx<T>* src = stage + ((size_t)g << LOGN) + i;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = src[t * TPL];
         }
-        const bool ok = mbar_wait_bounded(&bars[st], (unsigned)(j >> 1) & 1u, P.wait_cycles);
+        if (!P.shared) fence_async_smem(); // this thread's reads of the stage, before the next load's writes
         if (!__syncthreads_and(ok)) {
-            if (tid == 0) {
-                atomicExch(J.err, 1);
-                if (kn < P.nitems) mbar_wait_bounded(&bars[st ^ 1], (unsigned)((j + 1) >> 1) & 1u, P.wait_cycles);
-            }
+            if (tid == 0) atomicExch(J.err, 1);
             failed = true;
             break;
         }
-        cx<T>* buf = stage0 + (size_t)st * S * blk;
+        if (tid == 0 && !P.shared && kn < P.nitems) issue(kn); // every thread has read the stage
         const size_t row0 = (size_t)k * blk;
-        cx<T> v[8];
+        if (mode & RM_INV) line_fft<T, LOGN, 1>(v, line, i, tw, sync);
+        const size_t gline = (size_t)gs * J.N + row0 + ((size_t)(g - gs * L) << LOGN) + i; // element t at + t TPL
+        if constexpr (S == 1) { // the thread's elements are its points
+            if (mode & (RM_INV | RM_REND | RM_OBS | RM_RSTART | RM_PHI))
+                nd_row_points<T, D, LEAN, SL::count, TPL>(J, v, gline, mode, obs, acc,
+                                                            (mode & RM_PHI) ? cline + PL::pad(i) : nullptr,
+                                                            [](int t) { return PL::pad_step(t); });
+        } else if (mode & (RM_INV | RM_REND | RM_OBS | RM_RSTART | RM_PHI)) { // per-point stages in natural order
+            if (mode & RM_INV) sync(); // the line's last exchange has been read
+            {
+                cx<T>* d = line + PL::pad(i);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = buf[ix.at(g, i + (r << logm))];
-        if (mode & RM_INV) ndt_fft<T, 1>(v, buf, ix, logn, twm);
-        cx<T> w[8]; // RM_PHI: the end-of-step state, for its forward transform into phi
-        if (mode & (RM_INV | RM_REND | RM_OBS | RM_RSTART | RM_PHI)) { // per-point stages in natural order
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < 8; ++r) buf[ix.at(g, i + (r << logm))] = v[r];
-            __syncthreads();
-            constexpr uint32_t OBSMAX = POP ? (uint32_t)(WM_POP | WM_NORM) : ~0u;
-            if (PHI) { // end of step i, the copy, then the start of step i+1
-                nd_row_sweep<T, D, S, SL::count, IxRow<T>, OBSMAX>(J, buf, (cx<T>*)nullptr, ix, L, row0,
-                                                                   mode & ~(uint32_t)RM_RSTART, P.obs, acc);
-#pragma unroll
-                for (int r = 0; r < 8; ++r) w[r] = buf[ix.at(g, i + (r << logm))];
-                if (mode & RM_RSTART) {
-                    __syncthreads();
-                    nd_row_sweep<T, D, S, SL::count, IxRow<T>, OBSMAX>(J, buf, (cx<T>*)nullptr, ix, L, row0, RM_RSTART, 0u,
-                                                                       acc, false);
-                }
-            } else {
-                nd_row_sweep<T, D, S, SL::count, IxRow<T>, OBSMAX>(J, buf, (cx<T>*)nullptr, ix, L, row0, mode, P.obs, acc);
+                for (int t = 0; t < 16; ++t) d[PL::pad_step(t)] = v[t];
             }
-            if (mode & (RM_FWD | RM_STORE))
+            __syncthreads();
+            nd_row_sweep<T, D, S, LEAN, SL::count>(
+                J, exch, (mode & RM_PHI) ? copy : (cx<T>*)nullptr,
+                [ldx = P.ldx](int ln, int x) { return ln * ldx + PL::pad(x); }, L, row0, mode, obs, acc);
+            if (mode & (RM_FWD | RM_STORE)) {
+                const cx<T>* d = line + PL::pad(i);
 #pragma unroll
-                for (int r = 0; r < 8; ++r) v[r] = buf[ix.at(g, i + (r << logm))];
+                for (int t = 0; t < 16; ++t) v[t] = d[PL::pad_step(t)];
+            }
         }
-        if (mode & RM_FWD) ndt_fft<T, -1>(v, buf, ix, logn, twm);
+        if (mode & RM_FWD) {
+            sync();
+            line_fft<T, LOGN, -1>(v, line, i, tw, sync);
+        }
         if (mode & RM_STORE) {
-            __syncthreads();
+            cx<T>* dst = J.psi + gline;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) buf[ix.at(g, i + (r << logm))] = v[r];
-            fence_async_smem();
-            __syncthreads();
-            if (tid == 0) {
-                for (int s = 0; s < S; ++s) {
-                    const size_t row = ((size_t)s * J.N + row0) * sizeof(cx<T>) / 128;
-                    for (unsigned y = 0; y < rows_state; y += rows_box)
-                        tma_store_3d(&map, 0, (int)(row + y), 0,
-                                     reinterpret_cast<unsigned char*>(buf) + ((size_t)s * rows_state + y) * 128);
-                }
-                bulk_commit();
-            }
+            for (int t = 0; t < 16; ++t) dst[t * TPL] = v[t];
         }
-        if (PHI) { // forward transform of the end-of-step copy, through the same stage, into phi
-            if (tid == 0) bulk_wait_read_all(); // the psi store has read the stage
-            ndt_fft<T, -1>(w, buf, ix, logn, twm);
-            __syncthreads();
+        if (mode & RM_PHI) { // forward transform of the end-of-step copy into phi
+            const cx<T>* d = cline + PL::pad(i);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) buf[ix.at(g, i + (r << logm))] = w[r];
-            fence_async_smem();
+            for (int t = 0; t < 16; ++t) v[t] = d[PL::pad_step(t)];
+            sync();
+            line_fft<T, LOGN, -1>(v, cline, i, tw, sync);
+            cx<T>* dst = J.phi + gline;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) dst[t * TPL] = v[t];
+        }
+        if (P.shared) {
+            fence_async_smem(); // the exchange's writes, before the next load's
             __syncthreads();
-            if (tid == 0) {
-                for (int s = 0; s < S; ++s) {
-                    const size_t row = ((size_t)s * J.N + row0) * sizeof(cx<T>) / 128;
-                    for (unsigned y = 0; y < rows_state; y += rows_box)
-                        tma_store_3d(&map_phi, 0, (int)(row + y), 0,
-                                     reinterpret_cast<unsigned char*>(buf) + ((size_t)s * rows_state + y) * 128);
-                }
-                bulk_commit();
-            }
+            if (tid == 0 && kn < P.nitems) issue(kn);
+        } else if (S > 1) {
+            __syncthreads(); // the sweep of the next block reads and writes every line
+        } else {
+            sync();
         }
     }
-    if (tid == 0) bulk_wait_all();
     if (failed) return;
     if (sums) {
-        block_partials<SL::count>(acc, 0, J.part, J.nparts, part_base + blockIdx.x, act);
-        for (size_t col = blockIdx.x + gridDim.x; col < P.nitems; col += gridDim.x) // columns no CTA owns
+        __syncthreads();
+        cta_partials<SL::count>(acc, act, reinterpret_cast<double*>(exch), 0, J.part, J.nparts, part_base + blockIdx.x);
+        for (size_t col = blockIdx.x + P.workers; col < P.ncols; col += P.workers) // columns no CTA owns
             for (int v = tid; v < SL::count; v += blockDim.x) {
                 const size_t o = ((size_t)v * J.nparts + part_base + col) * 2;
                 J.part[o] = 0.0;
                 J.part[o + 1] = 0.0;
             }
     }
-    if (F.enabled && nd_last_cta(&F.book->counter, gridDim.x)) nd_finalize_cta(J, F);
+    if (F.enabled && nd_last_cta(&F.book->counter, P.workers)) nd_finalize_cta(J, F);
 }
 
 // per-axis kinetic phase exp(Complex(0, -k_i^2 / (2 m_j)) * dt) (Propagator.init, quantum_dynamics.zig:397-399)

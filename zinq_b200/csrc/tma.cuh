@@ -1,8 +1,8 @@
 // tma.cuh -- Tensor Memory Accelerator (TMA) staging for the N-D axis passes (sm_100a).
 //
-// Device side: mbarrier set-up and bounded waits, tiled tensor copies global -> shared
-// (completing on an mbarrier) and shared -> global (bulk groups).  Every copy here reads or
-// writes this GPU's own memory and none uses cluster multicast.
+// Device side: mbarrier set-up and bounded waits, tiled and untiled copies global -> shared
+// (completing on an mbarrier).  Every copy here reads this GPU's own memory and none uses cluster
+// multicast.
 // Host side: a tensor map over the wavefunction buffer, encoded through the driver entry point
 // that the runtime hands out (no link against libcuda).
 #pragma once
@@ -56,18 +56,13 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
-// tiled 3-D store of shared memory src to the box at (x, y, z), in the current bulk group
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z, const void* src) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
-                     reinterpret_cast<uint64_t>(map)),
-                 "r"(x), "r"(y), "r"(z), "r"(smem_u32(src))
+// untiled load of `bytes` contiguous bytes (a multiple of 16; both addresses 16-byte aligned); the
+// bytes complete on bar
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// the bulk groups committed by this thread have finished reading shared memory
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... and their writes to global memory are done
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -75,9 +70,8 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
 // ------------------------------------------------------------ host side
 // A 3-D tensor map of 8-byte words over `base`: dims[0] words fastest, then dims[1] rows at
 // stride1 bytes, dims[2] planes at stride2 bytes; box[3] words x rows x planes.  l2promo is
-// the L2 fill granularity in bytes (0, 64, 128 or 256); swizzle128: the 128-byte shared-memory
-// swizzle (box rows of exactly 128 bytes).  Returns a CUDA error code (as int): 0 on success.
+// the L2 fill granularity in bytes (0, 64, 128 or 256).  Returns a CUDA error code (as int): 0 on success.
 int encode_map_3d(CUtensorMap* map, void* base, const uint64_t dims[3], uint64_t stride1, uint64_t stride2,
-                  const uint32_t box[3], int l2promo, bool swizzle128 = false);
+                  const uint32_t box[3], int l2promo);
 
 } // namespace zqd
