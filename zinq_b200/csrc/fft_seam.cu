@@ -1,14 +1,18 @@
 // fft_seam.cu -- stand-alone N-D complex FFT of a device buffer (the FftPlan
-// seam, src/fourier_transform.zig:8-49).  Each CTA stages one line of one axis
-// in shared memory, runs the Stockham passes of the propagator kernels and
-// writes it back; the inverse applies the reference's 1/N afterwards.
+// seam, src/fourier_transform.zig:8-49).  Lines of 32 to 4096 points go through registers, sixteen
+// points a thread (nd_fft.cuh), a strided axis in tiles of neighbouring lines; shorter lines, lines of
+// 8192 points and the no-allocation variant stage one line per CTA in shared memory.  The inverse
+// applies the reference's 1/N.
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
 #include "line_kernel.cuh"
+#include "nd_fft.cuh"
 
 using namespace zqd;
 
@@ -16,7 +20,7 @@ struct zqd_fft {
     int ndim = 1, n = 0, sign = -1, logn = 0;
     size_t N = 0;
     bool fp32 = false;
-    void* tw = nullptr;
+    void* tw = nullptr; // exp(-2 pi i t / n), t < n, then the same pass by pass (LinePlan's table)
     ~zqd_fft() {
         if (tw) cudaFree(tw);
     }
@@ -41,6 +45,88 @@ template <typename T> __global__ void scale_kernel(cx<T>* data, size_t N, double
     if (i < N) data[i] = mk<T>((T)((double)data[i].x / (1.0 / s)), (T)((double)data[i].y / (1.0 / s)));
 }
 
+// One axis of the transform, W neighbouring lines of 2^LOGN points per group of threads: element t of
+// line g at base + t stride + g on a strided axis (ROW = false), at base + g n + t on the last.  The
+// elements go from global memory to registers and back; only the boundaries between the radix passes
+// use shared memory.  A warp takes whole lines up to 512 points (32/TPL of them: four 16-byte or four
+// 8-byte lines side by side at 128 points, one or two sectors a row) and waits for no other warp; a
+// CTA takes W lines above.  The twiddles (under 2 KB at 128 points, 31 KB at 2048) are read through
+// L1: staging them would cost each short CTA a wait.  Against one line per CTA with 16-byte accesses at
+// the axis stride, 128^3 FP64 227 -> 49 us forward (with the caller's copy of the
+// input), the three axes moving 201 MB through L2.
+template <typename T, int SIGN, int LOGN, bool ROW>
+__global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
+    fft_lines_kernel(cx<T>* __restrict__ data, int W, int logstride, int ldx, T scale_f, const Tab<T>* __restrict__ twd) {
+    using P = LinePlan<LOGN>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool WARP = P::TPL <= 32;
+    constexpr int LPW = WARP ? 32 / P::TPL : 1;
+    const int tid = threadIdx.x;
+    int g, i;
+    if constexpr (ROW) {
+        g = tid / P::TPL;
+        i = tid & (P::TPL - 1);
+    } else {
+        g = WARP ? (tid >> 5) * LPW + (tid & (LPW - 1)) : tid & (W - 1);
+        i = WARP ? (tid & 31) / LPW : tid / W;
+    }
+    const size_t l = (size_t)blockIdx.x * W + g; // the line
+    cx<T>* line = reinterpret_cast<cx<T>*>(smem_raw) + (size_t)g * ldx;
+    cx<T>* src;
+    if constexpr (ROW) src = data + (l << LOGN) + i;
+    else src = data + (((l >> logstride) << LOGN) << logstride) + (l & (((size_t)1 << logstride) - 1)) + ((size_t)i << logstride);
+    cx<T> v[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) v[t] = ROW ? src[t * P::TPL] : src[(size_t)(t * P::TPL) << logstride];
+    using SY = typename std::conditional<WARP, SyncWarp, SyncCta>::type;
+    line_fft<T, LOGN, SIGN>(v, line, i, twd, SY{});
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        if (SIGN > 0) v[t] = scale<T>(v[t], scale_f);
+        (ROW ? src[t * P::TPL] : src[(size_t)(t * P::TPL) << logstride]) = v[t];
+    }
+}
+
+template <typename T> using LinesKernel = void (*)(cx<T>*, int, int, int, T, const Tab<T>*);
+template <typename T, int LOGN = 5> static LinesKernel<T> lines_kernel(int logn, int sign, bool row) {
+    if constexpr (LOGN > 12) {
+        return nullptr;
+    } else {
+        if (logn != LOGN) return lines_kernel<T, LOGN + 1>(logn, sign, row);
+        if (row) return sign < 0 ? fft_lines_kernel<T, -1, LOGN, true> : fft_lines_kernel<T, 1, LOGN, true>;
+        return sign < 0 ? fft_lines_kernel<T, -1, LOGN, false> : fft_lines_kernel<T, 1, LOGN, false>;
+    }
+}
+
+// Lines per CTA: four warps' worth of short lines (fewer where the grid has fewer); above 512 points
+// one contiguous line, or the tile of strided lines that 256 threads (512 at 4096 points) hold.
+static int lines_per_cta(int logn, bool row, size_t lines) {
+    const int tpl = (1 << logn) / 16;
+    if (tpl > 32) return row ? 1 : logn == 12 ? 2 : 256 / tpl;
+    int w = 128 / tpl;
+    while ((size_t)w > lines || w * tpl > 128) w >>= 1;
+    return w;
+}
+
+template <typename T> static int fft_lines_exec(zqd_fft* p, cx<T>* data, cudaStream_t st) {
+    const Tab<T>* twd = (const Tab<T>*)p->tw + p->n;
+    const size_t lines = p->N / p->n;
+    int logstride = 0;
+    for (int a = p->ndim - 1; a >= 0; --a, logstride += p->logn) {
+        const bool row = a == p->ndim - 1;
+        const int W = lines_per_cta(p->logn, row, lines), tpl = p->n / 16;
+        const int ldx = exch_stride<T>(p->logn, row ? 0 : tpl <= 32 ? 32 / tpl : W);
+        const size_t smem = (size_t)W * ldx * sizeof(cx<T>);
+        const LinesKernel<T> k = lines_kernel<T>(p->logn, p->sign, row);
+        if (smem > 48 * 1024) ZQD_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the inverse's 1/N on its last axis
+        const T f = a == 0 ? (T)(1.0 / (double)p->N) : (T)1;
+        k<<<(unsigned)(lines / W), W * tpl, smem, st>>>(data, W, logstride, ldx, f, twd);
+        ZQD_CUDA(cudaGetLastError());
+    }
+    return ZQD_OK;
+}
+
 extern "C" int zqd_fft_plan_create(uint32_t ndim, const int* shape, int sign, zqd_precision precision, zqd_fft** out) {
     if (!out || !shape) return fail(ZQD_ERR_INVALID_INPUT, "NULL ARGUMENT");
     *out = nullptr;
@@ -62,13 +148,17 @@ extern "C" int zqd_fft_plan_create(uint32_t ndim, const int* shape, int sign, zq
     p->fp32 = precision == ZQD_FP32_MIXED;
     std::vector<double> tw = twiddles_f64(n);
     if (p->fp32) {
-        std::vector<float4> f(n);
+        std::vector<float4> f(2 * (size_t)n);
         for (int t = 0; t < n; ++t) f[t] = mktab<float>(tw[2 * t], tw[2 * t + 1]);
+        dense_twiddles(p->logn, f.data(), f.data() + n);
         ZQD_CUDA(cudaMalloc(&p->tw, f.size() * sizeof(float4)));
         ZQD_CUDA(cudaMemcpy(p->tw, f.data(), f.size() * sizeof(float4), cudaMemcpyHostToDevice));
     } else {
-        ZQD_CUDA(cudaMalloc(&p->tw, tw.size() * sizeof(double)));
-        ZQD_CUDA(cudaMemcpy(p->tw, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
+        std::vector<double2> f(2 * (size_t)n);
+        for (int t = 0; t < n; ++t) f[t] = mktab<double>(tw[2 * t], tw[2 * t + 1]);
+        dense_twiddles(p->logn, f.data(), f.data() + n);
+        ZQD_CUDA(cudaMalloc(&p->tw, f.size() * sizeof(double2)));
+        ZQD_CUDA(cudaMemcpy(p->tw, f.data(), f.size() * sizeof(double2), cudaMemcpyHostToDevice));
     }
     *out = p.release();
     return ZQD_OK;
@@ -101,6 +191,8 @@ template <typename T> static int fft_exec(zqd_fft* p, void* data, cudaStream_t s
 extern "C" int zqd_fft_execute(zqd_fft* p, void* data, void* stream) {
     if (!p || !data) return fail(ZQD_ERR_INVALID_INPUT, "NULL ARGUMENT");
     cudaStream_t st = (cudaStream_t)stream;
+    // 16-byte aligned elements are what FP64 accesses need; FP32 ones are 8 bytes
+    if (p->logn >= 5 && p->logn <= 12) return p->fp32 ? fft_lines_exec<float>(p, (cx<float>*)data, st) : fft_lines_exec<double>(p, (cx<double>*)data, st);
     return p->fp32 ? fft_exec<float>(p, data, st) : fft_exec<double>(p, data, st);
 }
 
