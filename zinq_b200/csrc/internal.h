@@ -91,11 +91,27 @@ int build_potential(const Opts& o, PotStore& ps, cudaStream_t st = nullptr);
 // Twiddle tables exp(-2 pi i t / n), t < n, generated in long double and rounded.
 std::vector<double> twiddles_f64(int n);
 
+// Doubles a result owns, uninitialised until written (a vector would first write zeros over them).
+class HostDoubles {
+    std::unique_ptr<double[]> p_;
+    size_t n_ = 0;
+
+  public:
+    double* reset(size_t n) {
+        p_.reset(n ? new double[n] : nullptr);
+        n_ = n;
+        return p_.get();
+    }
+    const double* data() const { return p_.get(); }
+    size_t size() const { return n_; }
+    bool empty() const { return n_ == 0; }
+};
+
 struct SolveOut {
     size_t rows = 0;
     std::vector<double> hist; // rows x HC
     std::vector<double> fin;  // HC
-    std::vector<double> psi;  // S x N complex, natural order
+    HostDoubles psi;          // S x N complex, natural order
     std::vector<double> acfpad, sigma;
     std::vector<double> wfn; // write.wavefunction: rows x S x N complex, natural order
 };

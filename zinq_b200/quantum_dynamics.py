@@ -224,9 +224,9 @@ def _collect(res_ptr):
 def _attach_wavefunctions(res_ptr, obs, npoint_total, nstate):
     L = _abi.load()
     for s, ob in enumerate(obs):
-        buf = np.zeros(2 * nstate * npoint_total)
-        check(L.zqd_result_wavefunction(res_ptr, s, buf.ctypes.data_as(_abi.DP), buf.size))
-        ob.wavefunction = (buf[0::2] + 1j * buf[1::2]).reshape(nstate, npoint_total)
+        psi = np.empty((nstate, npoint_total), dtype=np.complex128)  # (re, im) pairs, as the library writes them
+        check(L.zqd_result_wavefunction(res_ptr, s, psi.ctypes.data_as(_abi.DP), 2 * psi.size))
+        ob.wavefunction = psi
 
 
 def _shape(opt):
