@@ -32,6 +32,9 @@ VARIANTS += [("nd_inst.cu", f"nd_{t[0]}{s}", [f"-DZQD_T={t}", f"-DZQD_S={s}", f"
 VARIANTS += [("nd_tile.cu", f"nd_tile_{t[0]}", [f"-DZQD_T={t}", f"-DZQD_ND_TILE_PER_SM=nd_tile_per_sm_{t[0]}",
                                                  f"-DZQD_ND_TILE_LAUNCH=nd_tile_launch_{t[0]}"])
              for t in ("double", "float")]
+# and so do the small grids' whole-step kernels (every state count in one unit)
+VARIANTS += [("nd_small.cu", f"nd_small_{t[0]}", [f"-DZQD_T={t}", f"-DZQD_ND_SMALL_LAUNCH=nd_small_launch_{t[0]}"])
+             for t in ("double", "float")]
 
 
 def _stale(target, deps):

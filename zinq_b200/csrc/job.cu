@@ -936,6 +936,7 @@ extern "C" int zqd_run(const zqd_options* opt, zqd_result** out) {
     zqd_job* J = nullptr;
     int rc = zqd_job_create(opt, &J);
     if (rc) return rc;
+    J->nd_use_graph = false; // one run: its launches cost less than capturing them
     rc = zqd_job_run(J);
     if (!rc) rc = zqd_job_result(J, out);
     zqd_job_destroy(J);

@@ -115,6 +115,7 @@ struct zqd_job {
     bool nd_row_tma = false, nd_row_shared = true;
     int nd_row_tma_logL = 0, nd_row_tma_ctas = 0, nd_row_phi_ctas = 0;
     int nd_row_cols = 0, nd_k_cols = 0; // partial-sum columns of a row launch and of a momentum launch
+    bool nd_small = false; // 2-D grids of at most 128^2 points: whole steps in one cluster (nd_small.h), where the job's options allow
     cudaGraphExec_t nd_graph = nullptr; // the whole N-D run, captured on its first call and replayed after
     bool nd_use_graph = true;           // false: launch directly (one-shot jobs skip the capture cost)
     float last_ms = 0;

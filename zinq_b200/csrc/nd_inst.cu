@@ -11,6 +11,7 @@
 
 #include "job.h"
 #include "nd_kernels.cuh"
+#include "nd_small.h"
 #include "nd_tile.h"
 
 #if !defined(ZQD_T) || !defined(ZQD_S) || !defined(ZQD_ND_CREATE) || !defined(ZQD_ND_RUN) || !defined(ZQD_ND_STEP)
@@ -449,6 +450,8 @@ int ZQD_ND_CREATE(zqd_job* J) {
     if ((rc = choose_row_tma(J, ov.tma_rows)) || (rc = setup_tma_shape(J, ov.tma_w))) return rc;
     // columns of the partial sums: one per CTA of a row launch or of a momentum launch
     J->nd_row_cols = J->nd_row_tma ? std::max(J->nd_row_tma_ctas, J->nd_row_phi_ctas) : (int)(N / n / L);
+    // a forced or tuned shape of the axis passes is theirs
+    J->nd_small = J->d == 2 && J->nd_tma && J->nd_row_tma && log2_of(n) <= ND_SMALL_LOGN_MAX && !ov.rows && !ov.tile && !ov.tma_rows && !ov.tma_w;
     J->nd_k_cols = J->nd_tma ? J->nd_tma_ctas : (int)(S * (N / n / Tn));
     const size_t nparts = 3 * (size_t)J->nd_row_cols + J->nd_k_cols + 1024;
     if ((rc = J->psi_save.alloc((size_t)S * N * c, J->stream))) return rc;
@@ -552,6 +555,32 @@ struct Seq {
     bool deferred(int s) const {
         const Opts& o = J->o;
         return o.imag_nstate && s == 0 && !o.has_cap && !o.pot_td && !J->wfn_hist.p;
+    }
+    // Small 2-D grids in real time that record nothing in momentum space, track no absorption and keep no
+    // wavefunction history run whole ranges of steps in one launch (nd_small.h).
+    bool small() const {
+        const Opts& o = J->o;
+        return J->nd_small && !split && !o.log && !J->wfn_hist.p && !(o.has_cap && o.cap_track) &&
+               !(o.write_mask & (WM_MOM | WM_EKIN | WM_ETOT));
+    }
+    int small_steps(int s, int i0, int i1) const {
+        NdSmall P{};
+        P.i0 = i0;
+        P.i1 = i1;
+        P.iters = iters;
+        P.mask = J->o.write_mask | (acf ? (uint32_t)WM_ACF : 0u);
+        P.ldx = tile_ldx(J->n, 1);
+        P.hist = hist(s);
+        P.hc = HC;
+        P.rows_out = rows_out(s);
+        return nd_small_launch<T>(S, Lc.D.logn, Lc.D, P, J->stream);
+    }
+    // rows i0 .. i1 of solve s
+    int steps(int s, int i0, int i1) {
+        if (small()) return small_steps(s, i0, i1);
+        for (int i = i0; i <= i1; ++i)
+            if (const int rc = step(s, i)) return rc;
+        return ZQD_OK;
     }
     // this solve's wavefunction history entry of step i (write.wavefunction), or null
     cx<T>* whist(int s, int i) const {
@@ -682,8 +711,7 @@ int enqueue(zqd_job* J) {
     int rc;
     for (int s = 0; s < J->nsolve; ++s) {
         if ((rc = q.prologue(s))) return rc;
-        for (int i = 0; i <= q.iters; ++i)
-            if ((rc = q.step(s, i))) return rc;
+        if ((rc = q.steps(s, 0, q.iters))) return rc;
         if ((rc = q.epilogue(s))) return rc;
     }
     return ZQD_OK;
@@ -708,8 +736,7 @@ int ZQD_ND_STEP(zqd_job* J, int s, int i0, int i1, int* rows, int* ended) {
     int rc;
     ZQD_CUDA(cudaEventRecord(J->ev0, J->stream));
     if (i0 == 0 && (rc = q.prologue(s))) return rc;
-    for (int i = i0; i <= i1; ++i)
-        if ((rc = q.step(s, i))) return rc;
+    if ((rc = q.steps(s, i0, i1))) return rc;
     if ((rc = q.Lc.flush())) return rc;
     // the steps first, then the copies into pageable memory (one queued behind the steps would wait
     // inside the driver, where it can hold up other threads' copies)

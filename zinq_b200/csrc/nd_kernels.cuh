@@ -812,13 +812,15 @@ __device__ __forceinline__ void nd_row_points(const NdJob<T>& J, cx<T> (&v)[16],
 // whole batch first (its loads would otherwise wait one after the other); several states keep one
 // point at a time within the registers, the next point's R (up to three states: six entries) loaded
 // ahead.  Returns after a barrier.  bx(line, x): where point x of line s L + l sits in buf (and phi_src).
-template <typename T, int D, int S, bool LEAN, int NV, typename BX>
+// nt, sync: the threads that sweep (0 .. nt - 1) and their barrier.
+template <typename T, int D, int S, bool LEAN, int NV, typename BX, typename SY = SyncCta>
 __device__ __forceinline__ void nd_row_sweep(const NdJob<T>& J, cx<T>* buf, cx<T>* phi_src, const BX& bx, int L, size_t row0,
-                                             uint32_t mode, uint32_t obs, double (&acc)[NV]) {
+                                             uint32_t mode, uint32_t obs, double (&acc)[NV], int nt = blockDim.x,
+                                             const SY& sync = SY{}) {
     constexpr int SB = S == 1 ? 4 : 1;
     constexpr bool AHEAD = S == 2 || S == 3;
     using Aux = NdAux<T, S, (SB > 1)>;
-    const int logn = J.logn, pts = L << logn, nt = blockDim.x;
+    const int logn = J.logn, pts = L << logn;
     const T inv_n = (T)(1.0 / (double)J.N);
     const double f = (mode & RM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
     const bool wout = !LEAN && J.wfn_out != nullptr;
@@ -853,7 +855,7 @@ __device__ __forceinline__ void nd_row_sweep(const NdJob<T>& J, cx<T>* buf, cx<T
             for (int s = 0; s < S; ++s) buf[bx(s * L + l, x)] = v[s];
         }
     }
-    __syncthreads();
+    sync();
 }
 
 // L rows of the last axis (all S states) per CTA:
