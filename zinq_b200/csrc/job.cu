@@ -224,6 +224,34 @@ template <typename T> static size_t cxsize() { return sizeof(cx<T>); }
 // faster than on 8, 1024 points on 4 CTAs 15 % faster than on 2); ZQD_LINE_CLUSTER forces C
 // (tuning sweeps).  Radix-8 kernels exist for 16-CTA clusters only (lines above 16384 points in
 // FP64, 32768 in FP32); radix-4-only kernels keep the instruction footprint small.
+// Shared memory after the tables, as far as the budget goes: a third wavefunction buffer where the
+// steps record momentum-space observables, and the ring of unreduced sums (up to 16 steps and 64 KB; a
+// single CTA 8 steps and 40 KB, so that small lines still share an SM).
+static void line_extra_smem(zqd_job* J, size_t budget) {
+    const Opts& o = J->o;
+    const size_t c = J->fp32 ? sizeof(cx<float>) : sizeof(cx<double>);
+    const size_t ldp = J->fp32 ? padded_len<float>(J->m) : padded_len<double>(J->m);
+    auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    J->smem = up(J->smem);
+    J->ring_off = J->ring_steps = J->alt_off = 0;
+    if (o.write_mask & (WM_MOM | WM_EKIN | WM_ETOT)) {
+        const size_t b = up((size_t)J->S * ldp * c);
+        if (J->smem + b <= budget) {
+            J->alt_off = (int)J->smem;
+            J->smem += b;
+        }
+    }
+    const bool acf = o.has_spectrum || (o.write_mask & ZQD_WRITE_ACF);
+    const size_t step = (size_t)line_ring_values(o.write_mask, J->S, acf, o.has_cap && o.cap_track) * J->threads * sizeof(double2);
+    const size_t most = std::min<size_t>(J->C > 1 ? 64 * 1024 : 40 * 1024, budget - J->smem);
+    const size_t want = J->C > 1 ? RING_STEPS : RING_STEPS / 2, steps = step ? std::min(want, most / step) : want;
+    if (steps >= 2 && !(o.has_cap && o.cap_has_stop)) { // stop_norm needs each step's norm at once
+        J->ring_off = (int)J->smem;
+        J->ring_steps = (int)steps;
+        J->smem += steps * step;
+    }
+}
+
 static int choose_line_shape(zqd_job* J) {
     const size_t budget = 205 * 1024; // dynamic shared memory per CTA
     int forced = 0, forced_lr = 0;
@@ -269,6 +297,7 @@ static int choose_line_shape(zqd_job* J) {
             J->E = 8 * J->S;
             J->threads = threads;
             J->smem = u_smem ? smem_u : smem;
+            line_extra_smem(J, budget);
             J->r_global = rg;
             J->lrmax = lrmax;
             J->u_smem = u_smem;
@@ -416,6 +445,7 @@ template <typename T> static LineJob<T> line_job_desc(const zqd_job* J, int s) {
     L.logm = 0;
     while ((1 << L.logm) < J->m) ++L.logm;
     L.q = J->q;
+    L.nt = J->threads;
     L.lo = o.bounds[0];
     L.hi = o.bounds[1];
     L.dr = (o.bounds[1] - o.bounds[0]) / (double)o.npoint;
@@ -451,6 +481,9 @@ template <typename T> static LineJob<T> line_job_desc(const zqd_job* J, int s) {
     L.r_global = J->r_global ? 1 : 0;
     L.lrmax = J->lrmax;
     L.u_smem = J->u_smem ? 1 : 0;
+    L.ring_off = J->ring_off;
+    L.ring_steps = J->ring_steps;
+    L.alt_off = J->alt_off;
     L.sign_track = needs_sign_tracking(o, J->S, J->nsolve) ? 1 : 0;
     L.sgn = J->sgn.as<double>();
     L.wfn_hist = J->wfn_hist.p ? J->wfn_hist.as<cx<T>>() + (size_t)s * ((size_t)o.iterations + 1) * J->S * J->n : nullptr;

@@ -89,6 +89,7 @@ struct zqd_job {
     bool r_global = false; // 1-D: R read from global memory (the largest lines)
     int lrmax = 3;         // 1-D: log2 of the largest local radix
     bool u_smem = false;   // 1-D: the shape stages the eigenvectors in shared memory
+    int ring_off = 0, ring_steps = 0, alt_off = 0; // 1-D: shared memory after the tables (LineJob)
     int nsolve = 1, hc = 0;
     zqd::PotStore pot;
     cudaStream_t stream = nullptr;

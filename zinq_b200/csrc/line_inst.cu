@@ -45,6 +45,11 @@ static int launch_one(const LaunchShape* J, const void* d_jobs, int njobs) {
 // CTAs and 128 registers)
 template <int C> static int launch_r4(const LaunchShape* J, const void* dj, int nj) {
     if (LineMaxThreads<ZQD_T>::value > 256 && J->threads <= 256) return launch_one<C, 2, 256>(J, dj, nj);
+#if ZQD_S == 3
+    // three states on 512-point CTAs: 384 threads, 168 registers instead of 128
+    if constexpr (LineMaxThreads<ZQD_T>::value > 256)
+        if (J->threads <= 384) return launch_one<C, 2, 384>(J, dj, nj);
+#endif
     return launch_one<C, 2>(J, dj, nj);
 }
 

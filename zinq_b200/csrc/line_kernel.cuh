@@ -51,6 +51,7 @@ enum : uint32_t {
 
 template <typename T> struct LineJob {
     int n, m, logm, q;
+    int nt; // threads that work on the job (a group's launch may have more)
     double lo, hi, dr, dk, mass;
     int iters;
     double dt_re, dt_im, tstep;
@@ -77,6 +78,10 @@ template <typename T> struct LineJob {
     int r_global;          // R read from global memory instead of shared memory
     int lrmax;             // log2 of the largest local radix (threads per CTA = m >> lrmax)
     int u_smem;            // the shape reserved shared memory for the eigenvectors of the CTA's points
+    // dynamic shared memory after the tables (bytes from its start; 0: none): the ring of the rows'
+    // unreduced sums (ring_steps rows), and a third wavefunction buffer for steps that record
+    // momentum-space observables
+    int ring_off, ring_steps, alt_off;
     cx<T>* wfn_hist;       // [step][S][n] permuted wavefunction history of this solve, or null
     // time-dependent potentials whose eigenvector signs are observed (the adiabatic wavefunction
     // history, or the toDia of a later imaginary-time solve): after every update the 1-D
@@ -98,6 +103,7 @@ template <typename T> struct LineJob {
 };
 
 constexpr int NRED = 16;
+constexpr int RING_STEPS = 16; // most steps whose sums wait unreduced in the ring
 
 template <typename T> struct PadOf;
 template <> struct PadOf<double> { static constexpr int sh = 3; };
@@ -193,6 +199,8 @@ struct RedSmem {
     double slot[2][NRED][2];
     double res[NRED];
     int slot_idx; // alternates between the two cluster-visible slots
+    double2 w16[16];   // Tab<T> exp(-2 pi i e / 16) (16-CTA clusters)
+    double pop_abs[4]; // absorbed populations so far (thread 0's; CTA 0's are the solve's)
 };
 
 // Sums NV compensated accumulators over the cluster; every thread of every

@@ -11,7 +11,8 @@
 //   exchange      C-point DFTs across the cluster with the kinetic phase between them (C > 1)
 //   inverse FFT   first pass: remote gather of the exchanged values (C > 1), butterflies
 //                 last pass : butterflies, 1/N, [accumAbsorbed], psi <- R psi, observables
-// followed by one cluster reduction of the observables the step records.  The two
+// The observables' sums of up to 16 steps wait per thread in a ring in shared memory and are
+// reduced together (flush_rows).  The two
 // passes that apply R take all states of a butterfly in one thread; the other passes
 // and the exchange take one (butterfly or column, state) pair per thread.
 #pragma once
@@ -37,6 +38,13 @@ __host__ __device__ inline size_t line_smem_bytes(int S, int C, int m, bool r_gl
     const size_t ntw = line_two_schedules(m, lrm) ? 2 : 1;
     return 2 * (size_t)S * ld * sizeof(cx<T>) + ((C > 1 ? 1 : 0) + ntw + nsym + 1) * (size_t)m * sizeof(Tab<T>) +
            (u_smem ? (size_t)S * S * m * sizeof(double) : 0);
+}
+
+// Values a regular step of a job sums (the ring holds one (sum, compensation) pair of each per thread)
+inline int line_ring_values(uint32_t wmask, int S, bool acf, bool track) {
+    const bool ekin = wmask & (WM_EKIN | WM_ETOT), epot = wmask & (WM_EPOT | WM_ETOT);
+    return ((wmask & WM_NORM) ? 1 : 0) + ((wmask & WM_POS) ? 1 : 0) + (epot ? 1 : 0) + (acf ? 2 : 0) + ((wmask & WM_MOM) ? 1 : 0) +
+           (ekin ? 1 : 0) + ((wmask & WM_POP) ? S : 0) + (track ? S : 0);
 }
 
 // reduction slots of a step
@@ -448,6 +456,102 @@ __host__ __device__ __forceinline__ int local_pass_lr(int logm, int lrm, int idx
     return idx == (inverse ? np - 1 : 0) ? logm - (np - 1) * lrm : lrm;
 }
 
+// system-scope release store / acquire load: the host polls and writes these words in pinned memory
+__device__ __forceinline__ void st_release_sys(int* p, int v) {
+    asm volatile("st.release.sys.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.sys.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Reduces and writes the rows waiting in the ring: one warp per (row, value) over the CTA's threads,
+// CTA 0 over the cluster, one thread per row.  ring: value idx of row k of thread t at
+// [(k rnact + idx) nt + t].  Fixed order, so the result does not depend on how many
+// rows wait.  rs->warp holds the CTA's (sum, compensation) pairs, then CTA 0's totals.
+// (A function of its own, out of line: it takes values, not the solver, which stays in registers.)
+template <typename T, int S, int C>
+__device__ __noinline__ void line_flush_rows(const LineJob<T>* J, RedSmem* rs, const double2* ring, int rfill, int rfirst, int rnact,
+                                             ObsFlags rf, int cta, double dr, double dk) {
+    constexpr int NV = NAcc<S>::value;
+    const int nt = J->nt, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, pairs = rfill * rnact;
+    double* part = &rs->warp[0][0][0];
+    double* tot = part + 2 * RING_STEPS * NV;
+    static_assert(3 * RING_STEPS * NAcc<4>::value <= 32 * NRED * 2, "the pairs and totals fit the scratch");
+    __syncthreads();
+    for (int pr = warp; pr < pairs; pr += nw) {
+        const double2* src = ring + (size_t)pr * nt;
+        Acc t;
+        for (int e = lane; e < nt; e += 32) {
+            const double2 x = src[e];
+            t.add(x.x);
+            t.c += x.y;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const double s2 = __shfl_down_sync(0xffffffffu, t.s, off), c2 = __shfl_down_sync(0xffffffffu, t.c, off);
+            t.add(s2);
+            t.c += c2;
+        }
+        if (lane == 0) {
+            part[2 * pr] = t.s;
+            part[2 * pr + 1] = t.c;
+        }
+    }
+    if constexpr (C > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    if (cta == 0) {
+        for (int pr = threadIdx.x; pr < pairs; pr += blockDim.x) {
+            Acc t;
+            if constexpr (C > 1) {
+                for (int cc = 0; cc < C; ++cc) {
+                    const double* rem = cg::this_cluster().map_shared_rank(&part[2 * pr], cc);
+                    t.add(rem[0]);
+                    t.c += rem[1];
+                }
+            } else {
+                t.s = part[2 * pr];
+                t.c = part[2 * pr + 1];
+            }
+            tot[pr] = t.value();
+        }
+        __syncthreads();
+        if (rf.track && threadIdx.x == 0) // absorbed populations up to each row, in place of the row's own
+            for (int k = 0; k < rfill; ++k)
+                for (int s = 0; s < S; ++s) {
+                    double* a = &tot[k * rnact + rnact - S + s];
+                    rs->pop_abs[s] += *a * dr;
+                    *a = rs->pop_abs[s];
+                }
+        __syncthreads();
+        constexpr RowLayout L{1, S};
+        if (threadIdx.x < rfill) {
+            const double* v = tot + threadIdx.x * rnact; // the values in slot order
+            double* dst = J->hist + (size_t)(rfirst + threadIdx.x) * L.width();
+            const double nanv = nan("");
+            dst[L.norm()] = rf.norm ? *v++ * dr : nanv;
+            dst[L.pos()] = rf.pos ? *v++ * dr : nanv;
+            dst[L.epot()] = rf.epot ? *v++ * dr : nanv;
+            dst[L.acf()] = rf.acf ? *v++ * dr : nanv;
+            dst[L.acf() + 1] = rf.acf ? *v++ * dr : nanv;
+            dst[L.mom()] = rf.mom ? *v++ * dk : nanv;
+            dst[L.ekin()] = rf.ekin ? *v++ * dk : nanv;
+            const double* ab = tot + threadIdx.x * rnact + rnact - S; // read only with track
+            for (int s = 0; s < S; ++s) // not tracked: pop_abs is what an earlier launch carried (0)
+                dst[L.pop() + s] = rf.pop ? *v++ * dr + (rf.track ? ab[s] : 0.0) : nanv;
+        }
+        __syncthreads();
+        if (J->progress && threadIdx.x == 0) { // the rows are in memory: publish them to the host
+            __threadfence_system();
+            st_release_sys(J->progress, rfirst + rfill);
+        }
+    }
+    // nobody overwrites its pairs (or the ring) before they have been read
+    if constexpr (C > 1) cluster_barrier_relaxed();
+    else __syncthreads();
+}
+
 // All state of one CTA's solve.  Every member function is force-inlined into
 // the kernel, so the members stay in registers (no closure objects, no stack).
 template <typename T, int S, int C, int LRM> struct LineSolver {
@@ -472,6 +576,7 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
     const double* Vg;
     const cx<T>* psi0;
     int m, n, logm, q, ldp, cta;
+    int nt, tid0; // threads of the job; this thread's index, or past every loop's end
     size_t base;
     double lo, span, dr, dk, dkunit, mass;
     T inv_n;
@@ -479,7 +584,16 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
     bool fuse_obs; // accumulate the position-space observables in the last inverse pass
     ObsFlags f;
     Acc acc[NV];
-    double pop_abs[S];
+    int rfill; // rows waiting in the ring (their layout: line_flush_rows)
+
+    // what few places need is read from shared memory there, not kept in registers
+    __device__ __forceinline__ cx<T>* alt() const { // third wavefunction buffer, or null
+        return J->alt_off ? reinterpret_cast<cx<T>*>(reinterpret_cast<unsigned char*>(bufA) + J->alt_off) : nullptr;
+    }
+    __device__ __forceinline__ double2* ring() const {
+        return reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(bufA) + J->ring_off);
+    }
+    __device__ __forceinline__ Tab<T> w16(int e) const { return reinterpret_cast<const Tab<T>*>(rs->w16)[e]; }
 
     // ---------------------------------------------------------------- hooks
     // forward, first pass: accumAbsorbed before the first applyR, then R
@@ -560,13 +674,13 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
     __device__ __forceinline__ void pass(const cx<T>* __restrict__ in, cx<T>* __restrict__ out, int p,
                                          const cx<T>* xbuf) {
         constexpr int LR = R == 2 ? 1 : R == 4 ? 2 : 3;
-        const int logmr = logm - LR, mr = 1 << logmr, nt = blockDim.x;
+        const int logmr = logm - LR, mr = 1 << logmr;
         // passes whose hooks do not mix states take one (butterfly, state) pair per thread;
         // the forward first pass (R) and the inverse last pass (R, observables) take all
         // states of a butterfly in one thread
         constexpr bool SPLIT = S > 1 && !(KIND & FWD_FIRST) && !(KIND & INV_LAST);
         if constexpr (SPLIT) {
-            for (int t = threadIdx.x; t < (S << logmr); t += nt) {
+            for (int t = tid0; t < (S << logmr); t += nt) {
                 const int s = t >> logmr, i = t & (mr - 1);
                 cx<T> v[R];
                 if constexpr ((KIND & INV_FIRST) && C > 1) {
@@ -606,7 +720,7 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
             __syncthreads();
             return;
         }
-        for (int i = threadIdx.x; i < mr; i += nt) {
+        for (int i = tid0; i < mr; i += nt) {
             cx<T> v[S][R];
             if constexpr ((KIND & INV_FIRST) && C > 1) {
                 inv_first<R>(i, mr, v, xbuf);
@@ -677,10 +791,11 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
 
     // local m-point transform ping-ponging between a (input) and b; returns the result buffer.
     // start: passes already run (1: the first pass ran as part of the previous step's last pass);
-    // fuse_next (inverse only): the last pass also runs the next step's forward first pass
+    // fuse_next (inverse only): the last pass also runs the next step's forward first pass.
+    // c: with it the passes after the first ping-pong between b and c, and a keeps its contents
     template <int SIGN>
     __device__ __forceinline__ cx<T>* local_fft(cx<T>* a, cx<T>* b, const cx<T>* xbuf, int start = 0,
-                                                bool fuse_next = false) {
+                                                bool fuse_next = false, cx<T>* c = nullptr) {
         const int np = local_passes(logm, LRM);
         const Tab<T>* tw = SIGN < 0 ? twm : twi;
         int p = 1, tbase = 0;
@@ -703,7 +818,7 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
                 // gathered values were consumed (butterflies, stored locally) before the arrive,
                 // so the barrier publishes nothing and its arrive can be relaxed (no fence)
                 if (C > 1 && SIGN > 0 && first) cluster_barrier_relaxed();
-                cx<T>* t = in;
+                cx<T>* t = first && c ? c : in;
                 in = out;
                 out = t;
             }
@@ -717,29 +832,103 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
 
     __device__ __forceinline__ cx<T>* other(const cx<T>* b) const { return b == bufA ? bufB : bufA; }
 
+    __device__ __forceinline__ int logq() const { return logm - (C == 16 ? 4 : C == 8 ? 3 : C == 4 ? 2 : C == 2 ? 1 : 0); }
+    // C-point DFTs across the cluster over column (u, s), the kinetic phase or the momentum sums, and
+    // (propagation) the inverse DFTs into xb.  Up to 8 CTAs: one thread per column.
+    __device__ __forceinline__ void exchange(const cx<T>* res, cx<T>* xb) {
+        for (int t = tid0; t < S * q; t += nt) {
+            const int s = t >> logq(), u = t & (q - 1);
+            cx<T> w[C];
+#pragma unroll
+            for (int cc = 0; cc < C; ++cc) w[cc] = remote<T>(res, cc)[s * ldp + padx<T>(cta * q + u)];
+            dft<C, -1, T>(w);
+#pragma unroll
+            for (int k2 = 0; k2 < C; ++k2) {
+                if (prop) w[k2] = tmul<-1>(w[k2], eks[k2 * q + u]);
+                else observe_k1<T>(acc, w[k2], cta * q + u + m * k2, n, dkunit, mass, f);
+            }
+            if (!prop && alt()) continue;
+            dft<C, 1, T>(w);
+#pragma unroll
+            for (int cc = 0; cc < C; ++cc) xb[s * ldp + padx<T>(cc * q + u)] = w[cc];
+        }
+    }
+    // 16 CTAs: four threads per column and four values a thread, 16 = 4 x 4 with the two digits exchanged
+    // through the column's sixteen entries of xb.  One thread per column left two of eight warps at work
+    // for 2350 of a step's 20000 cycles (8192 points x 2 states FP32).
+    // Forward over j = j1 + 4 j2 to k = k2 + 4 k1, inverse back; entry k2 4 + j1, then (in place) j.
+    __device__ __forceinline__ void exchange16(const cx<T>* res, cx<T>* xb) {
+        const int items = 4 * S * q;
+        auto split = [&](int t, int& s, int& h, int& u) {
+            u = t & (q - 1);
+            const int r = t >> logq();
+            h = r & 3;
+            s = r >> 2;
+        };
+        for (int t = tid0; t < items; t += nt) {
+            int s, j1, u;
+            split(t, s, j1, u);
+            cx<T> w[4];
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) w[j2] = remote<T>(res, j1 + 4 * j2)[s * ldp + padx<T>(cta * q + u)];
+            dft<4, -1, T>(w);
+            cx<T>* x = xb + s * ldp;
+            x[padx<T>(j1 * q + u)] = w[0];
+#pragma unroll
+            for (int k2 = 1; k2 < 4; ++k2) x[padx<T>((k2 * 4 + j1) * q + u)] = tmul<-1>(w[k2], w16(j1 * k2));
+        }
+        __syncthreads();
+        for (int t = tid0; t < items; t += nt) {
+            int s, k2, u;
+            split(t, s, k2, u);
+            cx<T>* x = xb + s * ldp;
+            cx<T> w[4];
+#pragma unroll
+            for (int j1 = 0; j1 < 4; ++j1) w[j1] = x[padx<T>((k2 * 4 + j1) * q + u)];
+            dft<4, -1, T>(w);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) {
+                const int k = k2 + 4 * k1;
+                if (prop) w[k1] = tmul<-1>(w[k1], eks[k * q + u]);
+                else observe_k1<T>(acc, w[k1], cta * q + u + m * k, n, dkunit, mass, f);
+            }
+            if (!prop && alt()) continue;
+            dft<4, 1, T>(w);
+            x[padx<T>(k2 * 4 * q + u)] = w[0];
+#pragma unroll
+            for (int j1 = 1; j1 < 4; ++j1) x[padx<T>((k2 * 4 + j1) * q + u)] = tmul<1>(w[j1], w16(j1 * k2));
+        }
+        if (!prop && alt()) return;
+        __syncthreads();
+        for (int t = tid0; t < items; t += nt) {
+            int s, j1, u;
+            split(t, s, j1, u);
+            cx<T>* x = xb + s * ldp;
+            cx<T> w[4];
+#pragma unroll
+            for (int k2 = 0; k2 < 4; ++k2) w[k2] = x[padx<T>((k2 * 4 + j1) * q + u)];
+            dft<4, 1, T>(w);
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) x[padx<T>((j1 + 4 * j2) * q + u)] = w[j2];
+        }
+    }
+
     // forward transform of cur (start = 1: its first pass already ran); returns the buffer the
-    // inverse starts from
+    // inverse starts from.  With a third buffer a momentum observation (prop false) leaves cur as it
+    // is and needs no inverse.
     __device__ __forceinline__ cx<T>* forward(int start = 0) {
-        cx<T>* res = local_fft<-1>(cur, other(cur), nullptr, start);
+        cx<T>* res = local_fft<-1>(cur, other(cur), nullptr, start, false, prop ? nullptr : alt());
         if constexpr (C > 1) { // C-point DFTs across the cluster, kinetic phase in between
-            cx<T>* xb = other(res);
+            // a buffer that holds neither res nor (an observation with a third buffer) psi
+            cx<T>* xb = prop || !alt() ? other(res) : res == alt() ? other(cur) : alt();
             cg::cluster_group cl = cg::this_cluster();
             cl.sync();
-            // one (column u, state s) pair per thread: S times the threads of one column each
-            for (int t = threadIdx.x; t < S * q; t += blockDim.x) {
-                const int s = t / q, u = t - s * q;
-                cx<T> w[C];
-#pragma unroll
-                for (int cc = 0; cc < C; ++cc) w[cc] = remote<T>(res, cc)[s * ldp + padx<T>(cta * q + u)];
-                dft<C, -1, T>(w);
-#pragma unroll
-                for (int k2 = 0; k2 < C; ++k2) {
-                    if (prop) w[k2] = tmul<-1>(w[k2], eks[k2 * q + u]);
-                    else observe_k1<T>(acc, w[k2], cta * q + u + m * k2, n, dkunit, mass, f);
-                }
-                dft<C, 1, T>(w);
-#pragma unroll
-                for (int cc = 0; cc < C; ++cc) xb[s * ldp + padx<T>(cc * q + u)] = w[cc];
+            if constexpr (C == 16) exchange16(res, xb);
+            else exchange(res, xb);
+            if (!prop && alt()) {
+                // every CTA has read the others' buffers before the next step writes them
+                cluster_barrier_relaxed();
+                return nullptr;
             }
             cl.sync();
             return xb;
@@ -759,17 +948,19 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
     }
     // position-space observables of cur in a pass of their own
     __device__ __forceinline__ void observe_x() {
-        for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        for (int j = tid0; j < m; j += nt) {
             cx<T> x[S];
 #pragma unroll
             for (int s = 0; s < S; ++s) x[s] = cur[s * ldp + padx<T>(j)];
             observe_point<T, S>(acc, x, grid_r<C>(lo, span, n, cta, j), *J, base + j, f, Ug, ustride, j);
         }
     }
-    // momentum-space round trip (quantum_dynamics.zig:347-363): psi <- IFFT(FFT(psi)) as in the reference
+    // momentum-space observables (quantum_dynamics.zig:347-363).  The reference transforms psi and back;
+    // with a third buffer psi is kept instead of transformed back (a rounding's difference).
     __device__ __forceinline__ void roundtrip() {
         prop = false;
-        inverse(forward());
+        cx<T>* kb = forward();
+        if (!alt()) inverse(kb);
         prop = true;
     }
     __device__ __forceinline__ void set_flags(uint32_t mask) {
@@ -783,19 +974,46 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
         f.adia = J->adiabatic != 0;
         f.track = J->track != 0;
     }
+    // the values a step with these flags accumulates (the observe_* helpers add to no other slot)
+    __device__ __forceinline__ uint32_t act_mask(const ObsFlags& g) const {
+        uint32_t act = (g.norm ? 1u << A_NORM : 0u) | (g.pos ? 1u << A_POS : 0u) | (g.epot ? 1u << A_EPOT : 0u) |
+                       (g.acf ? 3u << A_ACFR : 0u) | (g.mom ? 1u << A_MOM : 0u) | (g.ekin ? 1u << A_EKIN : 0u);
+        if (g.pop) act |= ((1u << S) - 1u) << A_POP;
+        if (g.track) act |= ((1u << S) - 1u) << (A_POP + S);
+        return act;
+    }
+    // The sums of row i into the ring; a full ring is reduced.  Reducing every step's sums at once (a
+    // shuffle tree per value, then the warps, then the cluster, one thing after the other) was 23 % of
+    // a step: 4550 of 20000 cycles at 8192 points x 2 states, 1840 of 8200 at 256 points.
+    __device__ __forceinline__ void defer_row(int i) {
+        const uint32_t act = act_mask(f);
+        double2* dst = ring() + (size_t)rfill * __popc(act) * nt + threadIdx.x;
+        if ((int)threadIdx.x < nt)
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                if ((act >> v) & 1u) {
+                    *dst = make_double2(acc[v].s, acc[v].c);
+                    dst += nt;
+                }
+        if (++rfill == J->ring_steps) flush_rows(i);
+    }
+    // the waiting rows, the last of them row `last`
+    __device__ __forceinline__ void flush_rows(int last) {
+        if (rfill == 0) return;
+        const ObsFlags now = f;
+        set_flags(J->wmask); // the flags of the rows in the ring
+        line_flush_rows<T, S, C>(J, rs, ring(), rfill, last + 1 - rfill, __popc(act_mask(f)), f, cta, dr, dk);
+        f = now;
+        rfill = 0;
+    }
     // reduce the step's accumulators; the row is written by one thread of the cluster
     __device__ __forceinline__ double finish_row(double* dst) {
-        // the values this step accumulated (the observe_* helpers add to no other slot)
-        uint32_t act = (f.norm ? 1u << A_NORM : 0u) | (f.pos ? 1u << A_POS : 0u) | (f.epot ? 1u << A_EPOT : 0u) |
-                       (f.acf ? 3u << A_ACFR : 0u) | (f.mom ? 1u << A_MOM : 0u) | (f.ekin ? 1u << A_EKIN : 0u);
-        if (f.pop) act |= ((1u << S) - 1u) << A_POP;
-        if (f.track) act |= ((1u << S) - 1u) << (A_POP + S);
         double out[NV];
-        cluster_sum<NV, C>(acc, out, rs, act);
-#pragma unroll
-        for (int s = 0; s < S; ++s) pop_abs[s] += out[A_POP + S + s] * dr;
+        cluster_sum<NV, C>(acc, out, rs, act_mask(f));
         const double norm = out[A_NORM] * dr;
         if (cta == 0 && threadIdx.x == 0) {
+#pragma unroll
+            for (int s = 0; s < S; ++s) rs->pop_abs[s] += out[A_POP + S + s] * dr;
             constexpr RowLayout L{1, S};
             dst[L.norm()] = f.norm ? norm : nan("");
             dst[L.pos()] = f.pos ? out[A_POS] * dr : nan("");
@@ -805,21 +1023,11 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
             dst[L.mom()] = f.mom ? out[A_MOM] * dk : nan("");
             dst[L.ekin()] = f.ekin ? out[A_EKIN] * dk : nan("");
 #pragma unroll
-            for (int s = 0; s < S; ++s) dst[L.pop() + s] = f.pop ? out[A_POP + s] * dr + pop_abs[s] : nan("");
+            for (int s = 0; s < S; ++s) dst[L.pop() + s] = f.pop ? out[A_POP + s] * dr + rs->pop_abs[s] : nan("");
         }
         return norm;
     }
 };
-
-// system-scope release store / acquire load: the host polls and writes these words in pinned memory
-__device__ __forceinline__ void st_release_sys(int* p, int v) {
-    asm volatile("st.release.sys.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.sys.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 
 // The solve of job J (already in shared memory) on this CTA / cluster.
 template <typename T, int S, int C, int LRM>
@@ -834,6 +1042,8 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
     X.n = J.n;
     X.logm = J.logm;
     X.q = J.q;
+    X.nt = J.nt;
+    X.tid0 = (int)threadIdx.x < J.nt ? (int)threadIdx.x : 1 << 30;
     X.ldp = padded_len<T>(J.m);
     X.cta = cta;
     X.base = (size_t)cta * J.m;
@@ -866,8 +1076,9 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
     X.cur = X.bufA;
     X.prop = true;
     X.fuse_obs = false;
-#pragma unroll
-    for (int s = 0; s < S; ++s) X.pop_abs[s] = 0;
+    if constexpr (C == 16)
+        if (threadIdx.x < 16) reinterpret_cast<Tab<T>*>(rs.w16)[threadIdx.x] = J.tw[threadIdx.x * (J.n >> 4)];
+    X.rfill = 0;
 
     // stage the time-independent tables
     const int m = X.m, n = X.n;
@@ -912,6 +1123,8 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
     }
     __syncthreads();
 
+    if (threadIdx.x == 0)
+        for (int s = 0; s < S; ++s) rs.pop_abs[s] = J.i0 == 0 ? 0.0 : J.carry[s];
     LineCtx<T> ctx{&J, X.cur, nullptr, &rs, m, n, X.logm, X.q, X.ldp, cta, X.base};
     auto spare_of = [&](cx<T>* c) { return c == X.bufA ? X.bufB : X.bufA; };
     if (J.i0 == 0) {
@@ -921,8 +1134,6 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
             const int s = e / m, j = e - s * m;
             X.cur[s * X.ldp + padx<T>(j)] = J.psi_save[(size_t)s * n + X.base + j];
         }
-#pragma unroll
-        for (int s = 0; s < S; ++s) X.pop_abs[s] = J.carry[s];
         __syncthreads();
     }
     constexpr int HC = RowLayout{1, S}.width();
@@ -965,10 +1176,17 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
             X.roundtrip();
             ctx.psi = X.cur;
         }
-        const double nrm = X.finish_row(J.hist + (size_t)i * HC);
-        if (J.progress && cta == 0 && threadIdx.x == 0) { // row i is in memory: publish it to the host
-            __threadfence_system();
-            st_release_sys(J.progress, i + 1);
+        double nrm = 0; // read with has_stop only, whose rows are never deferred
+        // the ring takes the rows whose steps record what the write options ask for and nothing more
+        if (J.ring_steps && !logstep) {
+            X.defer_row(i);
+        } else {
+            X.flush_rows(i - 1);
+            nrm = X.finish_row(J.hist + (size_t)i * HC);
+            if (J.progress && cta == 0 && threadIdx.x == 0) { // row i is in memory: publish it to the host
+                __threadfence_system();
+                st_release_sys(J.progress, i + 1);
+            }
         }
         if (J.wfn_hist) { // History.append of the wavefunction (quantum_dynamics.zig:176-180), toAdia first (:919-927)
             cx<T>* __restrict__ dst = J.wfn_hist + (size_t)i * S * n;
@@ -1000,6 +1218,7 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
             break;
         }
     }
+    X.flush_rows(J.i1);
     if (ended) { // final Observables.init(..., log = true) (quantum_dynamics.zig:949)
         X.set_flags(WM_ALL_OBS);
         X.zero_acc();
@@ -1008,7 +1227,7 @@ __device__ __forceinline__ void line_solve_run(LineJob<T>& J, RedSmem& rs, unsig
         X.finish_row(J.fin);
     } else if (cta == 0 && threadIdx.x == 0) {
 #pragma unroll
-        for (int s = 0; s < S; ++s) J.carry[s] = X.pop_abs[s];
+        for (int s = 0; s < S; ++s) J.carry[s] = rs.pop_abs[s];
     }
     if (cta == 0 && threadIdx.x == 0) {
         *J.rows = rows;
