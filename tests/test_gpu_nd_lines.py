@@ -60,7 +60,8 @@ def test_3d_lines(n, S, precision):
 @pytest.mark.parametrize("rows,tile", [(1, 2), (4, 4), (8, 8), (32, 16)])
 @pytest.mark.parametrize("n,S", [(64, 2), (256, 1), (512, 3)])
 def test_shapes_at_the_edges_of_the_rules(tmp_path, n, S, rows, tile, precision):
-    # a tuning table forces the shape; one outside the kernel's limits is refused when the job is created
+    # a tuning table forces the shape (rounded up to whole warps of sixteen points a thread); one outside the
+    # kernel's limits is refused when the job is created
     table = tmp_path / "t.txt"
     table.write_text(f"2 {n} {S} {1 if precision == 'fp32' else 0} 0 0 0 0 {rows} {tile}\n")
     qd.tune_load(table)
@@ -72,7 +73,9 @@ def test_shapes_at_the_edges_of_the_rules(tmp_path, n, S, rows, tile, precision)
             return
         sh = j.nd_shape()
         j.close()
-        assert sh["tma_row_block"] == rows and sh["tma_tile_lines"] == tile
+        whole = lambda k, lines: k if lines * k * n // 16 % 32 == 0 else whole(2 * k, lines)  # noqa: E731
+        assert sh["tma_row_block"] == whole(rows, S) and sh["tma_tile_lines"] == whole(tile, 1)
+        assert sh["tma_row_threads"] % 32 == 0 and sh["tma_tile_threads"] % 32 == 0
         check(job(2, n, S, 4, "population norm"), precision)
     finally:
         qd.tune_clear()

@@ -946,7 +946,7 @@ extern "C" int zqd_job_nd_shape(const zqd_job* J, zqd_nd_shape* out) {
     *out = zqd_nd_shape{};
     if (J->nd_row_tma) {
         out->tma_row_block = 1u << J->nd_row_tma_logL;
-        out->tma_row_ctas = (uint32_t)J->nd_row_tma_ctas;
+        out->tma_row_ctas = (uint32_t)J->nd_row_ctas[1]; // the populations form
         out->tma_row_threads = (uint32_t)((size_t)J->S * J->n * out->tma_row_block / 16);
     }
     if (J->nd_tma) {

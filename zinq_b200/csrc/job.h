@@ -111,10 +111,10 @@ struct zqd_job {
     int nd_tma_logW = 0, nd_tma_ctas = 0;
     alignas(64) unsigned char nd_maps[2][128] = {};
     alignas(64) unsigned char nd_maps_phi[2][128] = {};
-    // the row pass's TMA-staged persistent form: rows per block (log2), CTAs of a launch without and
-    // with the momentum copy
-    bool nd_row_tma = false, nd_row_shared = true;
-    int nd_row_tma_logL = 0, nd_row_tma_ctas = 0, nd_row_phi_ctas = 0;
+    // the row pass's TMA-staged persistent form: rows per block (log2); per kernel form whether the stage
+    // and the exchange buffer share their space, and the CTAs; the CTAs of a launch with the momentum copy
+    bool nd_row_tma = false, nd_row_shared[4] = {true, true, true, true};
+    int nd_row_tma_logL = 0, nd_row_ctas[4] = {}, nd_row_phi_ctas = 0;
     int nd_row_cols = 0, nd_k_cols = 0; // partial-sum columns of a row launch and of a momentum launch
     bool nd_small = false; // 2-D grids of at most 128^2 points: whole steps in one cluster (nd_small.h), where the job's options allow
     cudaGraphExec_t nd_graph = nullptr; // the whole N-D run, captured on its first call and replayed after

@@ -144,19 +144,19 @@ struct Launch {
             P.obs = obs;
             P.logL = J->nd_row_tma_logL;
             P.nitems = (unsigned)(J->N / J->n >> P.logL);
-            P.workers = (unsigned)(phi ? J->nd_row_phi_ctas : J->nd_row_tma_ctas);
-            P.ncols = (unsigned)row_cols;
-            P.shared = phi || J->nd_row_shared;
-            P.ldx = row_ldx(J->n);
-            bool withhold = false;
-            P.wait_cycles = tma_wait_budget(NDT_WAIT_CYCLES, &withhold);
-            P.withhold = withhold;
-            const size_t smem = ndt_smem<T>(S << P.logL, J->n, P.ldx, P.shared, phi).total;
-            const unsigned nt = (unsigned)((S * J->n << P.logL) / 16);
             int form = RF_ALL;
             if (!(obs & ~row_form_obs(RF_POP))) form = RF_POP;
             else if (!(obs & ~row_form_obs(RF_ACF))) form = RF_ACF;
             if (d.track || d.wfn_out || (mode & RM_NORM)) form = RF_GENERAL;
+            P.workers = (unsigned)(phi ? J->nd_row_phi_ctas : J->nd_row_ctas[form]);
+            P.ncols = (unsigned)row_cols;
+            P.shared = phi || J->nd_row_shared[form];
+            P.ldx = row_ldx(J->n);
+            bool withhold = false;
+            P.wait_cycles = tma_wait_budget(NDT_WAIT_CYCLES, &withhold);
+            P.withhold = withhold;
+            const size_t smem = ndt_smem<T>(S << P.logL, J->n, P.ldx, P.shared, phi, row_ntw(form, J->n)).total;
+            const unsigned nt = (unsigned)((S * J->n << P.logL) / 16);
             const RowTmaKernel kern = row_tma(D.d, D.logn, form);
             kern<<<P.workers, nt, smem, J->stream>>>(d, P, region, f);
             ZQD_CUDA(cudaGetLastError());
@@ -202,7 +202,7 @@ struct Launch {
         P.nitems = (unsigned)S << P.logtiles;
         P.shared = J->nd_tma_shared;
         P.ldx = tile_ldx(J->n, 1 << P.logW);
-        const size_t smem = ndt_smem<T>(1 << P.logW, J->n, P.ldx, P.shared, false).total;
+        const size_t smem = ndt_smem<T>(1 << P.logW, J->n, P.ldx, P.shared, false, J->n).total;
         const unsigned threads = (unsigned)((J->n << P.logW) / 16);
         P.workers = (unsigned)J->nd_tma_ctas;
         if (phi) P.mode |= TM_PHI;
@@ -305,12 +305,13 @@ int setup_tma_shape(zqd_job* J, int w_override) {
     auto fits = [&](int W) {
         const size_t t = (size_t)W * n / 16;
         return W >= 1 && W <= n && (E * W) % 2 == 0 && t <= tmax && t % 32 == 0 &&
-               ndt_smem<T>(W, n, tile_ldx(n, W), true, false).total <= (size_t)ND_SMEM_BUDGET;
+               ndt_smem<T>(W, n, tile_ldx(n, W), true, false, n).total <= (size_t)ND_SMEM_BUDGET;
     };
     const size_t lines = J->N / (size_t)n; // lines of one state along any axis
     int W = 0;
     if (w_override > 0) W = w_override;
     if (W) {
+        while (W < n && (size_t)W * n / 16 % 32) W <<= 1; // whole warps (a table measured with eight points a thread)
         if (!fits(W) || lines % (size_t)W) return fail(ZQD_ERR_UNSUPPORTED, "TMA TILE SHAPE OUTSIDE THE KERNEL'S LIMITS");
     } else {
         // 64-byte rows, or 32-byte rows where that gives the device fewer than two tiles per SM (and the
@@ -322,7 +323,7 @@ int setup_tma_shape(zqd_job* J, int w_override) {
     const size_t items = (size_t)S * (lines / W);
     const int ldx = tile_ldx(n, W);
     int rc;
-    if ((rc = choose_grid(items, sms, 1, ndt_smem<T>(W, n, ldx, true, false).total, ndt_smem<T>(W, n, ldx, false, false).total,
+    if ((rc = choose_grid(items, sms, 1, ndt_smem<T>(W, n, ldx, true, false, n).total, ndt_smem<T>(W, n, ldx, false, false, n).total,
                           [&](size_t smem, int* per) { return nd_tile_per_sm<T>(d, logn, W * n / 16, smem, per); },
                           J->nd_tma_shared, J->nd_tma_ctas)))
         return rc;
@@ -371,28 +372,41 @@ int choose_row_tma(zqd_job* J, int l_override) {
     auto fits = [&](int L) {
         const size_t t = threads_of(L);
         return L >= 1 && (size_t)L <= lines && lines % (size_t)L == 0 && t % 32 == 0 && t <= (size_t)NDR_THREADS &&
-               ndt_smem<T>(S * L, n, ldx, true, true).total <= (size_t)ND_SMEM_BUDGET;
+               ndt_smem<T>(S * L, n, ldx, true, true, n).total <= (size_t)ND_SMEM_BUDGET;
     };
     int L = 0;
     if (l_override > 0) L = l_override;
     if (L) {
+        while ((size_t)L < lines && threads_of(L) % 32) L <<= 1; // whole warps (as for tiles)
         if (!fits(L)) return fail(ZQD_ERR_UNSUPPORTED, "TMA ROW-BLOCK SHAPE OUTSIDE THE KERNEL'S LIMITS");
-    } else { // the smallest block of at least 64 threads
+    } else { // the smallest block of at least 64 threads; one FP32 state 128 while the device has a block per SM
+        // (1024^2 28.3 -> 24.5 us a step, 128^3 49.0 -> 47.0; FP64 and several states lose: 128^3 x 2 FP64 134 -> 139)
         for (int l = 1; (size_t)l <= lines && !L; l <<= 1)
             if (fits(l) && (threads_of(l) >= 64 || !fits(2 * l))) L = l;
         if (!L) return ZQD_OK; // no shape fits: the earlier row kernel runs
+        if (S == 1 && sizeof(T) == 4 && fits(2 * L) && threads_of(2 * L) <= 128 && lines / (2 * L) >= (size_t)sms) L <<= 1;
     }
-    int rc;
-    bool shared_phi = true;
-    const size_t phi_smem = ndt_smem<T>(S * L, n, ldx, true, true).total; // the momentum copy always shares
-    auto per_sm = [&](size_t smem, int* per) -> int {
-        ZQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, (const void*)row_tma(d, logn, RF_ALL), (int)threads_of(L), smem));
-        return ZQD_OK;
-    };
-    if ((rc = choose_grid(lines / L, sms, 0, ndt_smem<T>(S * L, n, ldx, true, false).total,
-                          ndt_smem<T>(S * L, n, ldx, false, false).total, per_sm, J->nd_row_shared, J->nd_row_tma_ctas)) ||
-        (rc = choose_grid(lines / L, sms, 0, phi_smem, (size_t)ND_SMEM_BUDGET + 1, per_sm, shared_phi, J->nd_row_phi_ctas)))
-        return rc;
+    // each form's grid (their registers and twiddles differ), and the momentum copy's, which always shares
+    auto smem_of = [&](int form, bool shared, bool copy) { return ndt_smem<T>(S * L, n, ldx, shared, copy, row_ntw(form, n)).total; };
+    for (int form = 0; form <= RF_COUNT; ++form) {
+        const bool copy = form == RF_COUNT;
+        const int fk = copy ? (int)RF_ALL : form;
+        auto per_sm = [&](size_t smem, int* per) -> int {
+            ZQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, (const void*)row_tma(d, logn, fk), (int)threads_of(L), smem));
+            return ZQD_OK;
+        };
+        bool shared = true;
+        int ctas = 0;
+        if (const int rc = choose_grid(lines / L, sms, 0, smem_of(fk, true, copy),
+                                       copy ? (size_t)ND_SMEM_BUDGET + 1 : smem_of(fk, false, false), per_sm, shared, ctas))
+            return rc;
+        if (copy) {
+            J->nd_row_phi_ctas = ctas;
+        } else {
+            J->nd_row_ctas[form] = ctas;
+            J->nd_row_shared[form] = shared;
+        }
+    }
     J->nd_row_tma_logL = log2_of(L);
     J->nd_row_tma = true;
     return ZQD_OK;
@@ -449,7 +463,8 @@ int ZQD_ND_CREATE(zqd_job* J) {
     int rc;
     if ((rc = choose_row_tma(J, ov.tma_rows)) || (rc = setup_tma_shape(J, ov.tma_w))) return rc;
     // columns of the partial sums: one per CTA of a row launch or of a momentum launch
-    J->nd_row_cols = J->nd_row_tma ? std::max(J->nd_row_tma_ctas, J->nd_row_phi_ctas) : (int)(N / n / L);
+    J->nd_row_cols = (int)(N / n / L);
+    if (J->nd_row_tma) J->nd_row_cols = std::max(J->nd_row_phi_ctas, *std::max_element(J->nd_row_ctas, J->nd_row_ctas + RF_COUNT));
     // a forced or tuned shape of the axis passes is theirs
     J->nd_small = J->d == 2 && J->nd_tma && J->nd_row_tma && log2_of(n) <= ND_SMALL_LOGN_MAX && !ov.rows && !ov.tile && !ov.tma_rows && !ov.tma_w;
     J->nd_k_cols = J->nd_tma ? J->nd_tma_ctas : (int)(S * (N / n / Tn));

@@ -247,21 +247,25 @@ __device__ __forceinline__ double warp_sum_partials(const double* __restrict__ p
     const double2* __restrict__ src = reinterpret_cast<const double2*>(part) + (size_t)v * P;
     Acc t;
     size_t b = b0 + lane;
-    for (; b + 96 < b1; b += 128) { // four independent loads in flight
-        const double2 x0 = src[b], x1 = src[b + 32], x2 = src[b + 64], x3 = src[b + 96];
-        t.add(x0.x);
-        t.c += x0.y;
-        t.add(x1.x);
-        t.c += x1.y;
-        t.add(x2.x);
-        t.c += x2.y;
-        t.add(x3.x);
-        t.c += x3.y;
+    for (; b + 224 < b1; b += 256) { // eight independent loads in flight
+        double2 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = src[b + 32 * k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            t.add(x[k].x);
+            t.c += x[k].y;
+        }
     }
-    for (; b < b1; b += 32) {
-        const double2 x = src[b];
-        t.add(x.x);
-        t.c += x.y;
+    { // the last, at most eight: loaded together too
+        double2 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = b + 32 * k < b1 ? src[b + 32 * k] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            t.add(x[k].x);
+            t.c += x[k].y;
+        }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -394,7 +398,7 @@ template <typename T> __device__ void nd_finalize_cta(const NdJob<T>& J, const N
     }
     double* row = F.row;
     const RowLayout L{J.d, J.S};
-    if (F.kind == 0)
+    if (F.kind == 0 && J.track)
         for (int s = 0; s < J.S; ++s) { // accumAbsorbed adds sum * dr twice per step (quantum_dynamics.zig:497)
             book->pop_abs[s] += book->carry[s] * J.dr;
             book->pop_abs[s] += out[sl.abs() + s] * J.dr;
@@ -406,7 +410,7 @@ template <typename T> __device__ void nd_finalize_cta(const NdJob<T>& J, const N
         row[L.pos() + k] = c_pos ? out[sl.pos() + k] * J.dr : nan("");
         row[L.mom() + k] = c_mom ? out[sl.mom() + k] * J.dk : nan("");
     }
-    for (int s = 0; s < J.S; ++s) row[L.pop() + s] = c_pop ? out[sl.pop() + s] * J.dr + book->pop_abs[s] : nan("");
+    for (int s = 0; s < J.S; ++s) row[L.pop() + s] = c_pop ? out[sl.pop() + s] * J.dr + (J.track ? book->pop_abs[s] : 0.0) : nan("");
     row[L.epot()] = c_epot ? out[sl.epot()] * J.dr : nan("");
     row[L.ekin()] = c_ekin ? out[sl.ekin()] * J.dk : nan("");
     row[L.acf()] = c_acf ? out[sl.acf()] * J.dr : nan("");
@@ -1106,12 +1110,12 @@ constexpr long long NDT_WAIT_CYCLES = 4000000000LL; // ~2 s: a TMA load that has
 
 // shared memory of a TMA-staged pass of nl lines of n points: the stage, the exchange buffer (the
 // same space when shared), the row pass's copy of the end-of-step lines (momentum copies only), the
-// twiddles, the mbarriers, and slack to align the whole
+// twiddles (ntw entries, 0: read through L1), the mbarriers, and slack to align the whole
 struct NdtSmem {
     size_t stage, exch, copy, tw, bars, total;
 };
 template <typename T>
-__host__ __device__ inline NdtSmem ndt_smem(int nl, int n, int ldx, bool shared, bool copy) {
+__host__ __device__ inline NdtSmem ndt_smem(int nl, int n, int ldx, bool shared, bool copy, int ntw) {
     auto up = [](size_t b) { return (b + 127) & ~(size_t)127; };
     const size_t st = up((size_t)nl * n * sizeof(cx<T>)), ex = up((size_t)nl * ldx * sizeof(cx<T>));
     NdtSmem m;
@@ -1119,7 +1123,7 @@ __host__ __device__ inline NdtSmem ndt_smem(int nl, int n, int ldx, bool shared,
     m.exch = shared ? 0 : st;
     m.copy = shared ? (ex > st ? ex : st) : st + ex;
     m.tw = m.copy + (copy ? ex : 0);
-    m.bars = m.tw + (size_t)n * sizeof(Tab<T>);
+    m.bars = m.tw + (size_t)ntw * sizeof(Tab<T>);
     m.total = m.bars + 2 * sizeof(uint64_t) + 128;
     return m;
 }
@@ -1193,7 +1197,7 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     const int logW = P.logW, W = 1 << logW, tid = threadIdx.x;
-    const NdtSmem M = ndt_smem<T>(W, n, P.ldx, P.shared, false);
+    const NdtSmem M = ndt_smem<T>(W, n, P.ldx, P.shared, false, n);
     cx<T>* stage = reinterpret_cast<cx<T>*>(base + M.stage);
     cx<T>* exch = reinterpret_cast<cx<T>*>(base + M.exch);
     Tab<T>* tw = reinterpret_cast<Tab<T>*>(base + M.tw);
@@ -1369,6 +1373,11 @@ template <typename T> constexpr int row_bound(int S, int logn, int form) {
     return sizeof(T) == 8 ? (narrow ? 512 : 384) : narrow ? 608 : S <= 2 ? 512 : 416;
 }
 
+// Twiddles a row CTA stages: the narrow forms all; the wide ones, which the momentum copy takes, read them
+// through L1: without them four CTAs of a 512-point x 3-state FP64 row share an SM instead of three, and
+// 512 rows run at once instead of 444 and then 68 (total energy on 512^2 x 3: 52.9 -> 46.7 us a step).
+__host__ __device__ constexpr int row_ntw(int form, int n) { return form == RF_POP || form == RF_ACF ? n : 0; }
+
 template <typename T, int D, int S, int LOGN, int FORM>
 __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
     nd_row_tma_kernel(const __grid_constant__ NdJob<T> J, const NdRowTma P, size_t part_base,
@@ -1380,11 +1389,15 @@ __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     const int L = 1 << P.logL, tid = threadIdx.x;
     const uint32_t mode = P.mode;
-    const NdtSmem M = ndt_smem<T>(S * L, n, P.ldx, P.shared, mode & RM_PHI);
+    const NdtSmem M = ndt_smem<T>(S * L, n, P.ldx, P.shared, mode & RM_PHI, row_ntw(FORM, n));
     cx<T>* stage = reinterpret_cast<cx<T>*>(base + M.stage);
     cx<T>* exch = reinterpret_cast<cx<T>*>(base + M.exch);
     cx<T>* copy = reinterpret_cast<cx<T>*>(base + M.copy);
-    Tab<T>* tw = reinterpret_cast<Tab<T>*>(base + M.tw);
+    constexpr bool STAGED = row_ntw(FORM, n) > 0;
+    Tab<T>* tws = reinterpret_cast<Tab<T>*>(base + M.tw);
+    const Tab<T>* tw;
+    if constexpr (STAGED) tw = tws;
+    else tw = J.twd;
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + M.bars);
     const size_t blk = (size_t)L << LOGN; // points of one state in a block
     const unsigned sb = (unsigned)(blk * sizeof(cx<T>));
@@ -1402,7 +1415,8 @@ __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
     const int stopped = *J.stopped; // read beside the first load, not before it
     // the first load overlaps the twiddle staging (the stage and the twiddles do not overlap)
     if (tid == 0 && !P.withhold) issue(blockIdx.x);
-    for (int t = tid; t < PL::ntw; t += blockDim.x) tw[t] = J.twd[t];
+    if constexpr (STAGED)
+        for (int t = tid; t < PL::ntw; t += blockDim.x) tws[t] = J.twd[t];
     __syncthreads();
     const bool sums = mode & (RM_OBS | RM_REND | RM_RSTART);
     uint32_t act = 1u << SL::norm; // the slots this launch accumulates (nd_observe adds norm always)
