@@ -548,7 +548,7 @@ __device__ __noinline__ void line_flush_rows(const LineJob<T>* J, RedSmem* rs, c
         }
     }
     // nobody overwrites its pairs (or the ring) before they have been read
-    if constexpr (C > 1) cluster_barrier_relaxed();
+    if constexpr (C > 1) cg::this_cluster().sync();
     else __syncthreads();
 }
 
@@ -926,8 +926,10 @@ template <typename T, int S, int C, int LRM> struct LineSolver {
             if constexpr (C == 16) exchange16(res, xb);
             else exchange(res, xb);
             if (!prop && alt()) {
-                // every CTA has read the others' buffers before the next step writes them
-                cluster_barrier_relaxed();
+                // every CTA has read the others' buffers before the next step writes them: the ordered
+                // barrier, since up to 8 CTAs those reads end in registers only (exchange) and nothing
+                // else keeps them before the arrive
+                cl.sync();
                 return nullptr;
             }
             cl.sync();
