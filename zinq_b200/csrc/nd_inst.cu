@@ -206,6 +206,7 @@ struct Launch {
         const size_t smem = ndt_smem<T>(1 << P.logW, J->n, P.ldx, P.shared, false, J->n).total;
         const unsigned threads = (unsigned)((J->n << P.logW) / 16);
         P.workers = (unsigned)J->nd_tma_ctas;
+        P.ncols = (unsigned)row_cols;
         if (phi) P.mode |= TM_PHI;
         bool withhold = false;
         P.wait_cycles = tma_wait_budget(NDT_WAIT_CYCLES, &withhold);
@@ -223,12 +224,13 @@ struct Launch {
         if (mode & TM_KPHASE) std::swap(f, ahead);
         return tile_tma(axis, mode, false, 0, false, f);
     }
-    // forward along axes d-2..1, forward + kinetic phase + inverse along axis 0, inverse along 1..d-2
-    int step_tiles() {
+    // forward along axes d-2..1, forward + kinetic phase + inverse along axis 0, inverse along 1..d-2;
+    // `first`: mode bits of the first of these launches only (TM_SCALE, whose sum is region R0's)
+    int step_tiles(uint32_t first = 0) {
         int rc;
-        for (int a = D.d - 2; a >= 1; --a)
-            if ((rc = ptile(a, TM_FWD))) return rc;
-        if ((rc = ptile(0, TM_FWD | TM_KPHASE | TM_INV))) return rc;
+        for (int a = D.d - 2; a >= 1; --a, first = 0)
+            if ((rc = ptile(a, TM_FWD | first))) return rc;
+        if ((rc = ptile(0, TM_FWD | TM_KPHASE | TM_INV | first))) return rc;
         for (int a = 1; a <= D.d - 2; ++a)
             if ((rc = ptile(a, TM_INV))) return rc;
         return ZQD_OK;
@@ -568,8 +570,8 @@ struct Seq {
     // positions are quadratic in psi and the autocorrelation is linear, so the step closes and the
     // next one opens in a single row pass over the unnormalised psi, as in real time; its finalize
     // scales the observables row by the renormalisation factor (squared) and keeps the sum of
-    // |psi|^2, and the row pass that closes step i+1 (or the final observables' pass) multiplies psi
-    // by that factor.
+    // |psi|^2, and the first tile pass of step i+1 (or the final observables' pass) multiplies psi
+    // by that factor as it loads it.
     bool deferred(int s) const {
         const Opts& o = J->o;
         return o.imag_nstate && s == 0 && !o.has_cap && !o.pot_td && !J->wfn_hist.p;
@@ -661,10 +663,10 @@ struct Seq {
         const uint32_t obs = mask | ((o.has_cap && o.cap_has_stop) ? (uint32_t)WM_NORM : 0u);
         double* row = hist(s) + (size_t)i * HC;
         const bool defer = deferred(s);
-        if (i > 0 && (rc = Lc.step_tiles())) return rc;
+        if (i > 0 && (rc = Lc.step_tiles(defer ? (uint32_t)TM_SCALE : 0u))) return rc;
         if (!split || defer) {
             uint32_t mode = RM_OBS | RM_STORE | (needk ? RM_PHI : 0u);
-            if (i > 0) mode |= RM_INV | RM_REND | (defer ? (uint32_t)RM_SCALE : 0u);
+            if (i > 0) mode |= RM_INV | RM_REND;
             if (i < iters) mode |= RM_RSTART | RM_FWD;
             NdFin f = fin(s, 0, Lc.R0, Lc.R0 + Lc.row_cols, needk, mask, row, i);
             if (defer) f.nsum_out = Lc.scal();

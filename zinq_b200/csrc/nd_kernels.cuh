@@ -88,7 +88,7 @@ enum : uint32_t {
     RM_FWD = 1u << 5,    // forward FFT along the last axis
     RM_STORE = 1u << 6,  // write psi back
     RM_NORM = 1u << 7,   // after RM_REND: sum |psi|^2 into the norm slot (imaginary time: the renormalisation's norm)
-    RM_SCALE = 1u << 8,  // after the inverse transform: psi *= nd_norm_factor(*nsum, dr) (imaginary time)
+    RM_SCALE = 1u << 8,  // psi *= nd_norm_factor(*nsum, dr) before the other stages, in passes without RM_INV (imaginary time)
 };
 // tile-pass modes
 enum : uint32_t {
@@ -97,6 +97,7 @@ enum : uint32_t {
     TM_INV = 1u << 2,
     TM_KOBS = 1u << 3,   // after the forward FFT along axis 0: momentum observables, no store
     TM_PHI = 1u << 4,    // operate on phi instead of psi
+    TM_SCALE = 1u << 5,  // on load: psi *= nd_norm_factor(sum, dr) (imaginary time, renormalisation deferred)
 };
 
 // The renormalisation factor of psi whose sum of |psi|^2 is `sum`: 1 / sqrt(dr * sum), formed as
@@ -330,8 +331,8 @@ struct NdFin {
     NdBook* book;
     // kind 0, renormalisation deferred (imaginary time): the launch summed the unnormalised psi.
     // The row is scaled as if psi had been normalised first (every sum by the factor squared, the
-    // autocorrelation by the factor), and the raw sum of |psi|^2 goes to *nsum_out, where the row pass
-    // that closes the next step, or the final observables' pass, takes it from (RM_SCALE).
+    // autocorrelation by the factor), and the raw sum of |psi|^2 goes to *nsum_out, where the final
+    // observables' pass (RM_SCALE) and the per-block tile kernel (TM_SCALE) take it from.
     double* nsum_out;
     size_t x0, x1, k0, k1;
     double stop_norm;
@@ -1006,6 +1007,7 @@ __global__ void __launch_bounds__(512)
     const size_t outer = (size_t)blockIdx.x >> ltpo, inner0 = ((size_t)blockIdx.x & ((1u << ltpo) - 1)) << logt;
     const size_t c0 = ((outer << logn) << lstride) + inner0;
     cx<T>* data = ((mode & TM_PHI) ? J.phi : J.psi) + (size_t)blockIdx.y * J.N;
+    const double nf = (mode & TM_SCALE) ? nd_norm_factor(*J.nsum, J.dr) : 1.0;
     // element t of line g sits at data[c0 + (t << lstride) + g]; consecutive threads take consecutive lines
     cx<T> v[ND_IPT][8];
 #pragma unroll
@@ -1016,6 +1018,9 @@ __global__ void __launch_bounds__(512)
             nd_item<true>(it, logt, logm, g, i);
 #pragma unroll
             for (int r = 0; r < 8; ++r) v[k][r] = data[c0 + ((size_t)(i + (r << logm)) << lstride) + g];
+            if (mode & TM_SCALE)
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[k][r] = nd_scaled<T>(v[k][r], nf);
         }
     }
     __syncthreads(); // twiddles staged
@@ -1138,6 +1143,7 @@ struct NdTma {
     unsigned workers; // CTAs that take items
     int shared;      // the stage and the exchange buffer share their space
     int ldx;         // exchange line stride
+    unsigned ncols;  // TM_SCALE: columns of part (from 0) that hold the last row launch's norm sums
     long long wait_cycles; // budget of each mbarrier wait
     int withhold;    // testing: each CTA's first load is not issued, so its wait runs out
 };
@@ -1188,6 +1194,11 @@ __device__ __forceinline__ void cta_partials(const double (&a)[NV], uint32_t act
 // The stage holds element t of line g at t W + g, as the box lands.
 // TM_KOBS (the momentum observables of phi after its forward transform along axis 0) stores
 // nothing: its sums run over the CTA's tiles and are written once, at column blockIdx.x.
+// TM_SCALE (the first tile pass of an imaginary-time step): every CTA sums the norm's partials of the
+// row launch before it, in the same order, while its first tile is on the way, and normalises what it
+// loads.  Scaling later (in the row pass that closes the step, where the sum is known anyway) would let
+// two steps' factors exp(-E dt) act on the state before it is normalised, which FP32 does not hold for
+// wells far from the zero of energy.
 template <typename T, int D, int LOGN>
 __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     nd_tile_tma_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ CUtensorMap map, const NdTma P,
@@ -1235,7 +1246,13 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     // the first load overlaps the twiddle staging (the stage and the twiddles do not overlap)
     if (tid == 0 && !P.withhold) issue(blockIdx.x);
     for (int t = tid; t < PL::ntw; t += blockDim.x) tw[t] = J.twd[t];
+    __shared__ double norm_sum;
+    if ((P.mode & TM_SCALE) && tid < 32) {
+        const double x = warp_sum_partials(J.part, J.nparts, 0, P.ncols, Slots<D, 1>::norm);
+        if (tid == 0) norm_sum = x;
+    }
     __syncthreads();
+    const double nf = (P.mode & TM_SCALE) ? nd_norm_factor(norm_sum, J.dr) : 1.0;
     // the thread's line g of the tile and its place i in the line: a warp takes whole lines where
     // they are short enough, neighbouring threads neighbouring lines
     constexpr bool WARP = TPL <= 32;
@@ -1262,6 +1279,9 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
         if (ok) {
 #pragma unroll
             for (int t = 0; t < 16; ++t) v[t] = stage[((i + t * TPL) << logW) + g];
+            if (P.mode & TM_SCALE)
+#pragma unroll
+                for (int t = 0; t < 16; ++t) v[t] = nd_scaled<T>(v[t], nf);
         }
         if (!P.shared) fence_async_smem(); // this thread's reads of the stage, before the next load's writes
         if (!__syncthreads_and(ok)) { // the load never landed: record it and stop (none is in flight after it)
