@@ -22,7 +22,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxe
 SOURCES = ["options.cu", "expr.cpp", "job.cu", "result.cu", "fft_seam.cu", "spectrum.cu", "serve.cu", "tune.cu", "service.cu", "measure.cu", "tma_map.cu"]
 # line_inst.cu is compiled once per (precision, number of electronic states)
 VARIANTS = [("line_inst.cu", f"line_{t[0]}{s}", [f"-DZQD_T={t}", f"-DZQD_S={s}", f"-DZQD_LAUNCH=launch_line_{t[0]}{s}",
-                                                   f"-DZQD_SERVICE=launch_service_{t[0]}{s}"])
+                                                   f"-DZQD_SERVICE=launch_service_{t[0]}{s}", f"-DZQD_ROOM=line_room_{t[0]}{s}"])
             for t in ("double", "float") for s in (1, 2, 3, 4)]
 # nd_inst.cu likewise: the 2-D / 3-D driver
 VARIANTS += [("nd_inst.cu", f"nd_{t[0]}{s}", [f"-DZQD_T={t}", f"-DZQD_S={s}", f"-DZQD_ND_CREATE=nd_create_{t[0]}{s}",

@@ -224,32 +224,57 @@ template <typename T> static size_t cxsize() { return sizeof(cx<T>); }
 // faster than on 8, 1024 points on 4 CTAs 15 % faster than on 2); ZQD_LINE_CLUSTER forces C
 // (tuning sweeps).  Radix-8 kernels exist for 16-CTA clusters only (lines above 16384 points in
 // FP64, 32768 in FP32); radix-4-only kernels keep the instruction footprint small.
-// Shared memory after the tables, as far as the budget goes: a third wavefunction buffer where the
-// steps record momentum-space observables, and the ring of unreduced sums (up to 16 steps and 64 KB; a
-// single CTA 8 steps and 40 KB, so that small lines still share an SM).
-static void line_extra_smem(zqd_job* J, size_t budget) {
+int line_room_d1(const LaunchShape*, size_t*, size_t*);
+int line_room_d2(const LaunchShape*, size_t*, size_t*);
+int line_room_d3(const LaunchShape*, size_t*, size_t*);
+int line_room_d4(const LaunchShape*, size_t*, size_t*);
+int line_room_f1(const LaunchShape*, size_t*, size_t*);
+int line_room_f2(const LaunchShape*, size_t*, size_t*);
+int line_room_f3(const LaunchShape*, size_t*, size_t*);
+int line_room_f4(const LaunchShape*, size_t*, size_t*);
+
+// Shared memory after the tables, as far as the budget goes and as many CTAs share an SM as without it (the
+// kernel's registers allow one to four; with one less, a batch that fills the device takes more waves:
+// 296 jobs of 512 points x 2 states FP64 5.6 -> 8.9 ms): a third wavefunction buffer where the steps record
+// momentum-space observables (without it psi is transformed forward and back at such a step, as the
+// reference does: the results differ by the roundings of that pair), and the ring of unreduced sums (up
+// to 16 steps and 64 KB; a single CTA 8 steps and 40 KB).  The service kernel takes the same buffer and
+// as many of the ring's rows as leave its CTAs their places; a row's sums do not depend on how many wait.
+static int line_extra_smem(zqd_job* J, size_t budget) {
+    static int (*const dtab[4])(const LaunchShape*, size_t*, size_t*) = {line_room_d1, line_room_d2, line_room_d3, line_room_d4};
+    static int (*const ftab[4])(const LaunchShape*, size_t*, size_t*) = {line_room_f1, line_room_f2, line_room_f3, line_room_f4};
     const Opts& o = J->o;
     const size_t c = J->fp32 ? sizeof(cx<float>) : sizeof(cx<double>);
     const size_t ldp = J->fp32 ? padded_len<float>(J->m) : padded_len<double>(J->m);
     auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
     J->smem = up(J->smem);
-    J->ring_off = J->ring_steps = J->alt_off = 0;
+    J->ring_off = J->ring_steps = J->ring_service = J->alt_off = 0;
+    LaunchShape sh{J->S, J->C, J->E, J->threads, J->smem, nullptr};
+    sh.lrmax = J->lrmax;
+    size_t room = 0, svc = 0;
+    if (J->S < 1 || J->S > 4) return fail(ZQD_ERR_UNSUPPORTED, "STATE COUNT MUST BE 1..4");
+    if (const int rc = (J->fp32 ? ftab : dtab)[J->S - 1](&sh, &room, &svc)) return rc;
+    room = std::min(budget, room);
+    svc = std::min(budget, svc);
     if (o.write_mask & (WM_MOM | WM_EKIN | WM_ETOT)) {
         const size_t b = up((size_t)J->S * ldp * c);
-        if (J->smem + b <= budget) {
+        if (J->smem + b <= std::min(room, svc)) {
             J->alt_off = (int)J->smem;
             J->smem += b;
         }
     }
     const bool acf = o.has_spectrum || (o.write_mask & ZQD_WRITE_ACF);
     const size_t step = (size_t)line_ring_values(o.write_mask, J->S, acf, o.has_cap && o.cap_track) * J->threads * sizeof(double2);
-    const size_t most = std::min<size_t>(J->C > 1 ? 64 * 1024 : 40 * 1024, budget - J->smem);
+    const size_t most = std::min<size_t>(J->C > 1 ? 64 * 1024 : 40 * 1024, room > J->smem ? room - J->smem : 0);
     const size_t want = J->C > 1 ? RING_STEPS : RING_STEPS / 2, steps = step ? std::min(want, most / step) : want;
-    if (steps >= 2 && !(o.has_cap && o.cap_has_stop)) { // stop_norm needs each step's norm at once
+    // stop_norm needs each step's norm at once
+    if (steps >= 2 && J->smem + step <= svc && !(o.has_cap && o.cap_has_stop)) {
         J->ring_off = (int)J->smem;
         J->ring_steps = (int)steps;
+        J->ring_service = (int)(step ? std::min(steps, (svc - J->smem) / step) : steps);
         J->smem += steps * step;
     }
+    return ZQD_OK;
 }
 
 static int choose_line_shape(zqd_job* J) {
@@ -297,11 +322,10 @@ static int choose_line_shape(zqd_job* J) {
             J->E = 8 * J->S;
             J->threads = threads;
             J->smem = u_smem ? smem_u : smem;
-            line_extra_smem(J, budget);
             J->r_global = rg;
             J->lrmax = lrmax;
             J->u_smem = u_smem;
-            return ZQD_OK;
+            return line_extra_smem(J, budget);
         }
     }
     return fail(ZQD_ERR_UNSUPPORTED, "1-D GRID DOES NOT FIT THE RESIDENT CLUSTER KERNEL (at most 16 CTAs of 4096 points)");

@@ -90,6 +90,7 @@ struct zqd_job {
     int lrmax = 3;         // 1-D: log2 of the largest local radix
     bool u_smem = false;   // 1-D: the shape stages the eigenvectors in shared memory
     int ring_off = 0, ring_steps = 0, alt_off = 0; // 1-D: shared memory after the tables (LineJob)
+    int ring_service = 0; // rows of the ring in the service kernel (at most ring_steps)
     int nsolve = 1, hc = 0;
     zqd::PotStore pot;
     cudaStream_t stream = nullptr;

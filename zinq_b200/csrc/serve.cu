@@ -394,6 +394,10 @@ bool zqd_server::try_service(const Req& q) {
         return false;
     }
     J->fetch_psi = fetch_psi;
+    if (J->ring_steps > J->ring_service) {
+        J->smem = J->ring_off + (J->smem - J->ring_off) / J->ring_steps * J->ring_service;
+        J->ring_steps = J->ring_service;
+    }
     // the job's shape, rounded up: threads to a power of two (>= 64), shared memory to 16 KiB
     int threads = 64;
     while (threads < J->threads) threads <<= 1;
