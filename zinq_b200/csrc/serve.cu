@@ -110,8 +110,8 @@ struct SvcJob {
     int streamed = 0; // rows already posted as events
 };
 
-// service tables per (precision, states, threads per CTA, shared memory per CTA)
-using SvcKey = std::tuple<int, int, int, size_t>;
+// service tables per (precision, states, threads per CTA, shared memory per CTA, the part of it that the tables take)
+using SvcKey = std::tuple<int, int, int, size_t, size_t>;
 
 struct zqd_server {
     int device = 0;
@@ -402,8 +402,11 @@ bool zqd_server::try_service(const Req& q) {
     int threads = 64;
     while (threads < J->threads) threads <<= 1;
     const size_t smem = (J->smem + 16383) / 16384 * 16384;
+    // and of what its tables take alone: a class runs its jobs from one launch on, so two line lengths that meet in
+    // one only because of the memory taken after the tables stay apart
+    const size_t tables = J->alt_off ? J->alt_off : J->ring_off ? J->ring_off : J->smem;
     std::lock_guard<std::mutex> lk(svc_mu);
-    auto& host = svc[SvcKey{J->fp32 ? 1 : 0, J->S, threads, smem}];
+    auto& host = svc[SvcKey{J->fp32 ? 1 : 0, J->S, threads, smem, (tables + 16383) / 16384 * 16384}];
     if (!host) {
         host.reset(new zqd::LineServiceHost(J->fp32, J->S, threads, smem));
         if (host->init(1024, service_ctas, service_idle_us)) {
