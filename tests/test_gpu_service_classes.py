@@ -36,3 +36,29 @@ def test_lines_of_two_lengths_are_served_side_by_side():
     alone = served_ms([lines[2048]] * 8, "fp32")
     both = served_ms([lines[2048], lines[1024]] * 8, "fp32")
     assert both <= 1.3 * alone, (both, alone)
+
+
+@pytest.mark.parametrize("piece", [1, 4, 5])
+def test_rows_are_published_when_the_piece_asked_for_is_complete(piece):
+    # a ring of eight rows would publish counts that are multiples of eight only; a client that asks for smaller
+    # pieces gets them at other counts too (some 300 polls in 20 ms of steps; one in eight, four or eight of the
+    # counts are multiples of eight)
+    srv = qd.Server(workers=1, stream_steps=piece)
+    opt = small_line(1024, 1, 15.0, iters=3000)
+    opt["write"] = {"population": "P"}  # one value a row: a ring of eight rows
+    t = srv.submit(opt, "fp32")
+    firsts, rows, t0, done = [], [], time.time(), False
+    while not done:
+        for e in srv.poll():
+            done = done or e["kind"] == "done"
+            if e["kind"] == "rows":
+                firsts.append(e["first_row"])
+                rows.append(e["rows"])
+        assert time.time() - t0 < 60
+        time.sleep(0.0005)
+    r, _ = srv.wait(t)
+    srv.close()
+    assert any(f % 8 for f in firsts), firsts
+    got = np.concatenate(rows)
+    assert got.shape[0] == 3001
+    np.testing.assert_array_equal(got[:, 3:4], r.observables[0].history["population"])

@@ -394,9 +394,15 @@ bool zqd_server::try_service(const Req& q) {
         return false;
     }
     J->fetch_psi = fetch_psi;
-    if (J->ring_steps > J->ring_service) {
-        J->smem = J->ring_off + (J->smem - J->ring_off) / J->ring_steps * J->ring_service;
-        J->ring_steps = J->ring_service;
+    // rows wait in the kernel until its ring of them is full: no longer than leaves its CTAs their places and, where
+    // the client gets rows in pieces of stream_steps, in a length that divides a piece, so that
+    // every piece is published with its last row
+    if (J->ring_steps) {
+        int rows = J->ring_service;
+        if (stream_rows && stream_steps)
+            while (stream_steps % (uint32_t)rows) --rows;
+        J->smem = J->ring_off + (J->smem - J->ring_off) / J->ring_steps * rows;
+        J->ring_steps = rows;
     }
     // the job's shape, rounded up: threads to a power of two (>= 64), shared memory to 16 KiB
     int threads = 64;
