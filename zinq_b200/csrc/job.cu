@@ -238,8 +238,14 @@ int line_room_f4(const LaunchShape*, size_t*, size_t*);
 // 296 jobs of 512 points x 2 states FP64 5.6 -> 8.9 ms): a third wavefunction buffer where the steps record
 // momentum-space observables (without it psi is transformed forward and back at such a step, as the
 // reference does: the results differ by the roundings of that pair), and the ring of unreduced sums (up
-// to 16 steps and 64 KB; a single CTA 8 steps and 40 KB).  The service kernel takes the same buffer and
-// as many of the ring's rows as leave its CTAs their places; a row's sums do not depend on how many wait.
+// to 16 steps and 64 KB; a single CTA 8 steps and 40 KB).  Both may go 10 KB beyond the budget of the tables,
+// to what the launch allows: the longest lines' tables leave less than a row below it, and their steps
+// would each be reduced at once (32768 points FP64 16.8 us a step, with three rows 15.8).  A ring of one
+// row pays on CTAs of up to 256 threads (8192 points x 4 states FP64 with energies 33.9 -> 31.5 us a
+// step), not where its traffic does not: rows above 16 KB want three (8192 x 4 FP32: 27.3 us reduced at
+// once, 29.3 with two rows).
+// The service kernel takes the same buffer and as many of the ring's rows as leave its CTAs their places; a
+// row's sums do not depend on how many wait.
 static int line_extra_smem(zqd_job* J, size_t budget) {
     static int (*const dtab[4])(const LaunchShape*, size_t*, size_t*) = {line_room_d1, line_room_d2, line_room_d3, line_room_d4};
     static int (*const ftab[4])(const LaunchShape*, size_t*, size_t*) = {line_room_f1, line_room_f2, line_room_f3, line_room_f4};
@@ -254,6 +260,7 @@ static int line_extra_smem(zqd_job* J, size_t budget) {
     size_t room = 0, svc = 0;
     if (J->S < 1 || J->S > 4) return fail(ZQD_ERR_UNSUPPORTED, "STATE COUNT MUST BE 1..4");
     if (const int rc = (J->fp32 ? ftab : dtab)[J->S - 1](&sh, &room, &svc)) return rc;
+    budget += 10 * 1024;
     room = std::min(budget, room);
     svc = std::min(budget, svc);
     if (o.write_mask & (WM_MOM | WM_EKIN | WM_ETOT)) {
@@ -268,7 +275,7 @@ static int line_extra_smem(zqd_job* J, size_t budget) {
     const size_t most = std::min<size_t>(J->C > 1 ? 64 * 1024 : 40 * 1024, room > J->smem ? room - J->smem : 0);
     const size_t want = J->C > 1 ? RING_STEPS : RING_STEPS / 2, steps = step ? std::min(want, most / step) : want;
     // stop_norm needs each step's norm at once
-    if (steps >= 2 && J->smem + step <= svc && !(o.has_cap && o.cap_has_stop)) {
+    if (steps >= (step > 16384 ? 3u : J->threads > 256 ? 2u : 1u) && J->smem + step <= svc && !(o.has_cap && o.cap_has_stop)) {
         J->ring_off = (int)J->smem;
         J->ring_steps = (int)steps;
         J->ring_service = (int)(step ? std::min(steps, (svc - J->smem) / step) : steps);
