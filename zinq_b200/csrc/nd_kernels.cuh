@@ -816,14 +816,16 @@ __device__ __forceinline__ void nd_row_points(const NdJob<T>& J, cx<T> (&v)[16],
 // With one state a thread takes its points in batches of four and loads the global inputs of the
 // whole batch first (its loads would otherwise wait one after the other); several states keep one
 // point at a time within the registers, the next point's R (up to three states: six entries) loaded
-// ahead.  Returns after a barrier.  bx(line, x): where point x of line s L + l sits in buf (and phi_src).
+// ahead where NEXT says so: not in the per-block kernel, whose 512-thread form has no registers for it
+// (three states FP64: 480 bytes of spills became 1120, a step of 512^2 47 us became 60).
+// Returns after a barrier.  bx(line, x): where point x of line s L + l sits in buf (and phi_src).
 // nt, sync: the threads that sweep (0 .. nt - 1) and their barrier.
-template <typename T, int D, int S, bool LEAN, int NV, typename BX, typename SY = SyncCta>
+template <typename T, int D, int S, bool LEAN, bool NEXT, int NV, typename BX, typename SY = SyncCta>
 __device__ __forceinline__ void nd_row_sweep(const NdJob<T>& J, cx<T>* buf, cx<T>* phi_src, const BX& bx, int L, size_t row0,
                                              uint32_t mode, uint32_t obs, double (&acc)[NV], int nt = blockDim.x,
                                              const SY& sync = SY{}) {
     constexpr int SB = S == 1 ? 4 : 1;
-    constexpr bool AHEAD = S == 2 || S == 3;
+    constexpr bool AHEAD = NEXT && (S == 2 || S == 3);
     using Aux = NdAux<T, S, (SB > 1)>;
     const int logn = J.logn, pts = L << logn;
     const T inv_n = (T)(1.0 / (double)J.N);
@@ -916,7 +918,7 @@ __global__ void __launch_bounds__(MAXT)
         double acc[SL::count];
 #pragma unroll
         for (int q = 0; q < SL::count; ++q) acc[q] = 0.0;
-        nd_row_sweep<T, D, S, false, SL::count>(J, cur, (mode & RM_PHI) ? oth : (cx<T>*)nullptr,
+        nd_row_sweep<T, D, S, false, false, SL::count>(J, cur, (mode & RM_PHI) ? oth : (cx<T>*)nullptr,
                               [ldp](int line, int x) { return line * ldp + padx<T>(x); }, L, row0, mode, obs, acc);
         if (mode & (RM_OBS | RM_REND | RM_RSTART)) {
             // the slots this launch accumulates (nd_observe adds norm always, the rest by mask)
@@ -1500,7 +1502,7 @@ __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
                 for (int t = 0; t < 16; ++t) d[PL::pad_step(t)] = v[t];
             }
             __syncthreads();
-            nd_row_sweep<T, D, S, LEAN, SL::count>(
+            nd_row_sweep<T, D, S, LEAN, true, SL::count>(
                 J, exch, (mode & RM_PHI) ? copy : (cx<T>*)nullptr,
                 [ldx = P.ldx](int ln, int x) { return ln * ldx + PL::pad(x); }, L, row0, mode, obs, acc);
             if (mode & (RM_FWD | RM_STORE)) {

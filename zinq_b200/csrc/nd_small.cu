@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(S * 64 + 32, 1)
 #pragma unroll
                 for (int t = 0; t < 16; ++t) d[PL::pad_step(t)] = v[t];
                 all();
-                nd_row_sweep<T, 2, S, true, SL::count>(
+                nd_row_sweep<T, 2, S, true, true, SL::count>(
                     J, exch, (cx<T>*)nullptr, [ldx = P.ldx](int ln, int x) { return ln * ldx + PL::pad(x); }, L, row0, mode, P.mask,
                     acc, nt, all);
 #pragma unroll
