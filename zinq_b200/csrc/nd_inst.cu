@@ -89,7 +89,7 @@ NdJob<T> describe(zqd_job* J) {
 // and two 256-thread CTAs per SM hide more latency than extra registers would.
 inline bool row_narrow(unsigned threads) { return S > 1 && threads <= 256; }
 
-using RowTmaKernel = void (*)(NdJob<T>, NdRowTma, size_t, NdFin);
+using RowTmaKernel = void (*)(NdJob<T>, NdRowTma, size_t);
 // the longest line of the TMA-staged row pass: sixteen points a thread, at most 256 threads for the
 // states of one row, and no longer than the tile pass's
 constexpr int ROW_LOGN_MAX = S == 1 ? 12 : S == 2 ? 11 : 10;
@@ -123,15 +123,32 @@ struct Launch {
     size_t row_cols, k_cols; // partial-sum columns of a row launch and of a momentum launch
     // partial-sum regions (in blocks)
     size_t R0, R1, R2, K, G;
-    NdFin ahead{}; // sums waiting for the next tile launch's extra CTA (FIN_AHEAD), if enabled
+    NdFin ahead{}; // sums waiting for the next kinetic tile launch's extra CTA (FIN_AHEAD), if enabled
 
     // the waiting sums now, in a launch of their own
-    int flush() {
+    int flush(bool nostop = false) {
         if (!ahead.enabled) return ZQD_OK;
-        nd_finalize_kernel<T><<<1, 256, 0, J->stream>>>(D, ahead);
+        NdJob<T> d = D;
+        if (nostop) d.stopped = J->flags.as<int>() + 1; // a flag nothing sets
+        nd_finalize_kernel<T><<<1, 256, 0, J->stream>>>(d, ahead);
         ahead.enabled = 0;
         ZQD_CUDA(cudaGetLastError());
         return ZQD_OK;
+    }
+
+    // a row launch and, with momentum observables (RM_PHI), the launches that sum them, then the sums' reduction f:
+    // by the last CTA of a per-block launch, at once (now), or by the next kinetic tile launch.
+    int observe(uint32_t mode, uint32_t obs, size_t region, NdFin f, bool now, bool nostop = false, cx<T>* wout = nullptr) {
+        // (per-block launches on large grids: 64^3 26.8 us a step against 28.3 with nd_finalize_kernel, where 32^3, 16^3
+        // and 128^2 take 26.3, 24.6 and 21.1 with that against 27.3, 31.2 and 23.0)
+        const bool k = mode & RM_PHI, own = (k ? !J->nd_tma : !J->nd_row_tma) && J->N >= ((size_t)1 << 18);
+        int rc;
+        f.enabled = own ? FIN_LAST : FIN_AHEAD;
+        if ((rc = row(mode, obs, region, nostop, own && !k ? f : NdFin{}, wout))) return rc;
+        if (k && (rc = kobs(nostop, own ? f : NdFin{}))) return rc;
+        if (own) return ZQD_OK;
+        ahead = f;
+        return now ? flush(nostop) : ZQD_OK;
     }
 
     int row(uint32_t mode, uint32_t obs, size_t region, bool nostop = false, NdFin f = NdFin{}, cx<T>* wout = nullptr) {
@@ -159,7 +176,7 @@ struct Launch {
             const size_t smem = ndt_smem<T>(S << P.logL, J->n, P.ldx, P.shared, phi, row_ntw(form, J->n)).total;
             const unsigned nt = (unsigned)((S * J->n << P.logL) / 16);
             const RowTmaKernel kern = row_tma(D.d, D.logn, form);
-            kern<<<P.workers, nt, smem, J->stream>>>(d, P, region, f);
+            kern<<<P.workers, nt, smem, J->stream>>>(d, P, region);
             ZQD_CUDA(cudaGetLastError());
             return ZQD_OK;
         }
@@ -186,7 +203,8 @@ struct Launch {
         return ZQD_OK;
     }
     // the TMA-staged persistent form of a tile pass: over psi (modes TM_FWD, TM_KPHASE, TM_INV) or
-    // over phi (TM_FWD, or TM_FWD | TM_KOBS: the momentum sums into region `region`, finalized by f)
+    // over phi (TM_FWD, or TM_FWD | TM_KOBS: the momentum sums into region `region`)
+    // (f: an earlier launch's sums, for an extra CTA)
     int tile_tma(int axis, uint32_t mode, bool phi = false, size_t region = 0, bool nostop = false, NdFin f = NdFin{}) {
         NdJob<T> d = D;
         if (nostop) d.stopped = J->flags.as<int>() + 1;
@@ -259,13 +277,14 @@ struct Launch {
         ZQD_CUDA(cudaGetLastError());
         return ZQD_OK;
     }
-    // momentum observables of phi (the forward transform along the last axis is already done)
+    // momentum observables of phi (the forward transform along the last axis is already done); f: the
+    // per-block kernel's last CTA's reduction
     int kobs(bool nostop, NdFin f) {
         int rc;
         if (J->nd_tma) {
             for (int a = D.d - 2; a >= 1; --a)
                 if ((rc = tile_tma(a, TM_FWD, true, 0, nostop))) return rc;
-            return tile_tma(0, TM_FWD | TM_KOBS, true, K, nostop, f);
+            return tile_tma(0, TM_FWD | TM_KOBS, true, K, nostop);
         }
         for (int a = D.d - 2; a >= 1; --a)
             if ((rc = tile(a, TM_FWD | TM_PHI, 0, nostop))) return rc;
@@ -606,7 +625,7 @@ struct Seq {
     cx<T>* whist(int s, int i) const {
         return J->wfn_hist.p ? J->wfn_hist.as<cx<T>>() + ((size_t)s * (iters + 1) + i) * S * J->N : nullptr;
     }
-    // finalize descriptors, run by the last CTA of the launch that ends a step
+    // finalize descriptors
     NdFin fin(int s, int kind, size_t x0, size_t x1, bool k, uint32_t mask, double* row, int i) const {
         const Opts& o = J->o;
         NdFin f{};
@@ -622,7 +641,6 @@ struct Seq {
         f.row_index = i;
         f.kind = kind;
         f.has_stop = kind == 0 && o.has_cap && o.cap_has_stop;
-        f.enabled = FIN_LAST;
         return f;
     }
     int itp_ops(int s) { // quantum_dynamics.zig:898-906
@@ -671,11 +689,7 @@ struct Seq {
             NdFin f = fin(s, 0, Lc.R0, Lc.R0 + Lc.row_cols, needk, mask, row, i);
             if (defer) f.nsum_out = Lc.scal();
             const uint32_t o2 = obs | (defer ? (uint32_t)WM_NORM : 0u);
-            if ((rc = Lc.row(mode, o2, Lc.R0, false, NdFin{}, whist(s, i)))) return rc;
-            if (needk && (rc = Lc.kobs(false, NdFin{}))) return rc;
-            f.enabled = FIN_AHEAD; // by the next step's first tile launch
-            Lc.ahead = f;
-            return ZQD_OK;
+            return Lc.observe(mode, o2, Lc.R0, f, false, false, whist(s, i));
         }
         // Imaginary time, first state (nothing to orthogonalise against), no absorbing potential, after
         // step 0: the pass that closes step i also sums |psi|^2, and the next pass divides by the norm
@@ -692,20 +706,20 @@ struct Seq {
         if (o.pot_td && (rc = Lc.table((double)i * o.time_step, 0))) return rc;
         // R0 holds the end-of-step sums of the row pass that closed step i (none at i = 0)
         const NdFin f = fin(s, 0, i > 0 ? Lc.R0 : Lc.R1, Lc.R1 + Lc.row_cols, needk, mask, row, i);
+        // stop_norm decides before the next launch; tracked absorption's carry is replaced by that launch's sums
+        const bool track = Lc.D.track, now = f.has_stop || track;
         if (fuse && !o.pot_td && i < iters) { // normalise, observe, and open step i+1 in one pass
             const uint32_t mode = RM_SCALE | RM_OBS | RM_RSTART | RM_FWD | RM_STORE | (needk ? (uint32_t)RM_PHI : 0u);
-            if ((rc = Lc.row(mode, obs, Lc.R1, false, needk ? NdFin{} : f, whist(s, i)))) return rc;
-            if (needk && (rc = Lc.kobs(false, f))) return rc;
-            return ZQD_OK;
+            return Lc.observe(mode, obs, Lc.R1, f, now, false, whist(s, i));
         }
         const uint32_t omode = RM_OBS | (needk ? (uint32_t)RM_PHI : 0u) | (fuse ? (uint32_t)(RM_SCALE | RM_STORE) : 0u);
-        if ((rc = Lc.row(omode, obs, Lc.R1, false, needk ? NdFin{} : f, whist(s, i)))) return rc;
-        if (needk && (rc = Lc.kobs(false, f))) return rc;
+        if ((rc = Lc.observe(omode, obs, Lc.R1, f, now, false, whist(s, i)))) return rc;
         if (i < iters) {
             if (o.pot_td && (rc = Lc.table(((double)i + 0.5) * o.time_step, 1))) return rc;
+            const uint32_t mode = RM_RSTART | RM_FWD | RM_STORE;
+            if (!track) return Lc.row(mode, 0, Lc.R2);
             // the absorbed sums of step i+1's first accumAbsorbed
-            const NdFin fc = fin(s, 2, Lc.R2, Lc.R2 + Lc.row_cols, false, 0, nullptr, 0);
-            if ((rc = Lc.row(RM_RSTART | RM_FWD | RM_STORE, 0, Lc.R2, false, fc))) return rc;
+            return Lc.observe(mode, 0, Lc.R2, fin(s, 2, Lc.R2, Lc.R2 + Lc.row_cols, false, 0, nullptr, 0), false);
         }
         return ZQD_OK;
     }
@@ -716,8 +730,8 @@ struct Seq {
         const uint32_t all = WM_ALL_OBS | (acf ? (uint32_t)WM_ACF : 0u);
         // a deferred renormalisation (the last step's) is applied here, and psi stored normalised
         const uint32_t scale = deferred(s) ? (uint32_t)(RM_SCALE | RM_STORE) : 0u;
-        if ((rc = Lc.row(RM_OBS | RM_PHI | scale, all, Lc.R1, true))) return rc;
-        if ((rc = Lc.kobs(true, fin(s, 1, Lc.R1, Lc.R1 + Lc.row_cols, true, all, J->fin.as<double>() + (size_t)s * HC, 0))))
+        if ((rc = Lc.observe(RM_OBS | RM_PHI | scale, all, Lc.R1,
+                             fin(s, 1, Lc.R1, Lc.R1 + Lc.row_cols, true, all, J->fin.as<double>() + (size_t)s * HC, 0), true, true)))
             return rc;
         if (s + 1 < J->nsolve) // orthw.append (quantum_dynamics.zig:586-591)
             ZQD_CUDA(cudaMemcpyAsync(J->orth.as<char>() + (size_t)s * SN, J->psi_save.p, SN, cudaMemcpyDeviceToDevice, J->stream));

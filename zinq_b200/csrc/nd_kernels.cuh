@@ -316,11 +316,13 @@ struct NdBook {
     unsigned counter; // CTAs of the current launch that have written their partials
 };
 
-// What one CTA does with the partial sums of a row or momentum launch (enabled != 0): the last CTA of
-// that launch itself (FIN_LAST), where the host or the next launch needs the outcome at once
-// (stop_norm), or an extra CTA of the next tile launch (FIN_AHEAD), beside that launch's own work.
-// The reduction and the row's bookkeeping are a chain of dependent loads and sums, which at the end
-// of every step cost 2-4 us of a 13-60 us step.
+// What one CTA does with the partial sums of a row or momentum launch (enabled != 0).  After TMA-staged
+// launches that is an extra CTA of the next kinetic tile launch, beside that launch's own work
+// (FIN_AHEAD), or nd_finalize_kernel where the next launch needs the outcome (stop_norm, tracked
+// absorption) and at the end of a range of steps: the reduction and the row's bookkeeping are a chain of
+// dependent loads and sums, which at the end of every step cost 2-4 us of a 13-60 us step, and more in the
+// last CTA of such a launch, whose two to eight warps take one value each (512^2 x 2 FP32 with stop_norm:
+// 8-11 us of a launch of 28-31).  The last CTA of a per-block launch of many CTAs does it itself (FIN_LAST).
 // kind 0: the observables row of step row_index (plus absorbed bookkeeping and stop_norm);
 // kind 1: the final observables (no bookkeeping); kind 2: only record the absorbed sums
 // of the next step's first accumAbsorbed.  [x0, x1): position-space and absorbed partial
@@ -422,7 +424,7 @@ template <typename T> __device__ void nd_finalize_cta(const NdJob<T>& J, const N
     }
 }
 
-// the sums of an earlier launch when no tile launch follows that could take them along
+// the sums of an earlier launch where no kinetic tile launch can take them along
 template <typename T> __global__ void nd_finalize_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ NdFin F) {
     if (*J.stopped) return;
     nd_finalize_cta(J, F);
@@ -1348,7 +1350,6 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     __syncthreads();
     cta_partials<D + 1>(acc, (1u << (D + 1)) - 1u, reinterpret_cast<double*>(exch), Slots<D, 1>::mom, J.part, J.nparts,
                         part_base + blockIdx.x);
-    if (F.enabled == FIN_LAST && nd_last_cta(&F.book->counter, P.workers)) nd_finalize_cta(J, F);
 }
 
 // ------------------------------------------------------------ row pass, TMA-staged and persistent
@@ -1402,8 +1403,7 @@ __host__ __device__ constexpr int row_ntw(int form, int n) { return form == RF_P
 
 template <typename T, int D, int S, int LOGN, int FORM>
 __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
-    nd_row_tma_kernel(const __grid_constant__ NdJob<T> J, const NdRowTma P, size_t part_base,
-                      const __grid_constant__ NdFin F) {
+    nd_row_tma_kernel(const __grid_constant__ NdJob<T> J, const NdRowTma P, size_t part_base) {
     using SL = Slots<D, S>;
     using PL = LinePlan<LOGN>;
     constexpr int n = PL::n, TPL = PL::TPL;
@@ -1551,7 +1551,6 @@ __global__ void __launch_bounds__(row_bound<T>(S, LOGN, FORM), 1)
                 J.part[o + 1] = 0.0;
             }
     }
-    if (F.enabled && nd_last_cta(&F.book->counter, P.workers)) nd_finalize_cta(J, F);
 }
 
 // per-axis kinetic phase exp(Complex(0, -k_i^2 / (2 m_j)) * dt) (Propagator.init, quantum_dynamics.zig:397-399)
