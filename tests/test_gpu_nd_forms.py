@@ -6,7 +6,8 @@ points per axis up, and 3-D), so that every launch of a step is an axis pass.
   both, over different partitions of the same points).
 * The narrow forms against the oracle at the N-D parity bars (FP64 populations 1e-12, autocorrelation and
   other observables 1e-10; FP32 populations 1e-5, autocorrelation 1e-4).
-* Repeats are the same bit for bit; a TMA wait that runs out in the middle of a run fails the run."""
+* Repeats are the same bit for bit; a TMA wait that runs out in the middle of a run fails the run.
+* A tuned shape is accepted exactly where the passes' limits say so."""
 import copy
 
 import numpy as np
@@ -84,3 +85,43 @@ def test_a_wait_that_runs_out_between_steps_fails_the_run():
     j.close()
     opt = copy.deepcopy(pop_256(iters=6))  # the armed launch is used up: the next run is whole
     compare(opt)
+
+
+def tuned_job(tmp_path, n, S, rows, tile, precision):
+    table = tmp_path / "t.txt"
+    table.write_text(f"2 {n} {S} {1 if precision == 'fp32' else 0} 0 0 0 0 {rows} {tile}\n")
+    qd.tune_load(table)
+    try:
+        return qd.Job(job(2, n, S, 1, "population"), precision=precision)
+    finally:
+        qd.tune_clear()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("rows,tile", [(1, 2), (2, 8), (4, 4), (8, 8), (16, 16), (32, 16), (3, 0), (0, 3), (0, 16), (16, 0)])
+@pytest.mark.parametrize("n,S", [(8, 1), (16, 1), (16, 2), (32, 4), (64, 2), (256, 1), (512, 3), (2048, 2)])
+def test_tuned_shapes_are_accepted_within_the_limits(tmp_path, n, S, rows, tile, precision):
+    # whole warps of eight points a thread, at most 512 threads (rows of three and four states 256), blocks of at
+    # least 1024 bytes, tile rows of whole 16 bytes; grids below 32 points take the per-block kernels with any of these
+    c = 16 if precision == "fp64" else 8
+    warps = lambda points, most: points // 8 % 32 == 0 and points // 8 <= most  # noqa: E731
+    row_ok = rows == 0 or (n % rows == 0 and rows * n * c >= 1024 and warps(S * rows * n, 512 if S <= 2 else 256))
+    tile_ok = tile == 0 or (n % tile == 0 and tile * c % 16 == 0 and warps(tile * n, 512))
+    if not (row_ok and tile_ok):
+        with pytest.raises(_abi.ZqdError) as err:
+            tuned_job(tmp_path, n, S, rows, tile, precision)
+        assert err.value.status == -7
+        return
+    j = tuned_job(tmp_path, n, S, rows, tile, precision)
+    sh = j.nd_shape()
+    j.close()
+
+    def widened(k, lines):  # to whole warps of sixteen points a thread
+        while lines * k * n // 16 % 32:
+            k *= 2
+        return k
+
+    if rows:
+        assert sh["tma_row_block"] == (widened(rows, S) if n >= 32 else 0)
+    if tile:
+        assert sh["tma_tile_lines"] == (widened(tile, 1) if n >= 32 else 0)

@@ -310,6 +310,11 @@ int choose_grid(size_t items, int sms, int extra, size_t smem_shared, size_t sme
     return ZQD_OK;
 }
 
+// A table's or the autotuner's shape for the TMA-staged passes names whole warps of eight points a thread, the
+// threads these passes had when the first tables were measured, up to `most` of them; other shapes are
+// refused.  (Sixteen points a thread: blocks that leave half a warp are widened.)
+inline bool tuned_threads_ok(size_t points, size_t most) { return points / 8 % 32 == 0 && points / 8 <= most; }
+
 // The TMA-staged tile pass: lines per tile W (a power of two, W <= n) with rows of W c >= 16
 // bytes (an even number of 8-byte words), W n / 16 threads (whole warps, at most 256, 512 on lines of
 // 4096 points; a line of at most 512 points within one warp) and the stage, exchange and
@@ -321,7 +326,10 @@ int setup_tma_shape(zqd_job* J, int w_override) {
     const int n = J->n, d = J->d, logn = log2_of(n);
     J->nd_tma = false;
     const char* env = getenv("ZQD_ND_TMA");
-    if ((env && env[0] == '0') || w_override < 0 || logn < ND_TMA_LOGN_MIN || logn > nd_tma_logn_max<T>(d)) return ZQD_OK;
+    if ((env && env[0] == '0') || w_override < 0) return ZQD_OK;
+    if (w_override > 0 && (w_override > n || (E * w_override) % 2 || (J->N / n) % w_override || !tuned_threads_ok((size_t)w_override * n, 512)))
+        return fail(ZQD_ERR_UNSUPPORTED, "TMA TILE SHAPE OUTSIDE THE KERNEL'S LIMITS");
+    if (logn < ND_TMA_LOGN_MIN || logn > nd_tma_logn_max<T>(d)) return ZQD_OK; // the per-block kernels
     int dev = 0, sms = 148;
     ZQD_CUDA(cudaGetDevice(&dev));
     ZQD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -335,7 +343,7 @@ int setup_tma_shape(zqd_job* J, int w_override) {
     int W = 0;
     if (w_override > 0) W = w_override;
     if (W) {
-        while (W < n && (size_t)W * n / 16 % 32) W <<= 1; // whole warps (a table measured with eight points a thread)
+        while (W < n && (size_t)W * n / 16 % 32) W <<= 1; // whole warps
         if (!fits(W) || lines % (size_t)W) return fail(ZQD_ERR_UNSUPPORTED, "TMA TILE SHAPE OUTSIDE THE KERNEL'S LIMITS");
     } else {
         // 64-byte rows, or 32-byte rows where that gives the device fewer than two tiles per SM (and the
@@ -386,7 +394,11 @@ int choose_row_tma(zqd_job* J, int l_override) {
     const size_t lines = J->N / (size_t)n;
     J->nd_row_tma = false;
     const char* env = getenv("ZQD_ND_TMA");
-    if ((env && env[0] == '0') || l_override < 0 || logn < ND_TMA_LOGN_MIN || !row_tma(d, logn, RF_GENERAL)) return ZQD_OK;
+    if ((env && env[0] == '0') || l_override < 0) return ZQD_OK;
+    if (l_override > 0 && ((size_t)l_override > lines || lines % (size_t)l_override || (size_t)l_override * n * sizeof(cx<T>) < 1024 ||
+                           !tuned_threads_ok((size_t)S * l_override * n, S <= 2 ? 512 : 256)))
+        return fail(ZQD_ERR_UNSUPPORTED, "TMA ROW-BLOCK SHAPE OUTSIDE THE KERNEL'S LIMITS");
+    if (logn < ND_TMA_LOGN_MIN || !row_tma(d, logn, RF_GENERAL)) return ZQD_OK; // the per-block kernels
     int dev = 0, sms = 148;
     ZQD_CUDA(cudaGetDevice(&dev));
     ZQD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -401,7 +413,7 @@ int choose_row_tma(zqd_job* J, int l_override) {
     int L = 0;
     if (l_override > 0) L = l_override;
     if (L) {
-        while ((size_t)L < lines && threads_of(L) % 32) L <<= 1; // whole warps (as for tiles)
+        while ((size_t)L < lines && threads_of(L) % 32) L <<= 1; // whole warps
         if (!fits(L)) return fail(ZQD_ERR_UNSUPPORTED, "TMA ROW-BLOCK SHAPE OUTSIDE THE KERNEL'S LIMITS");
     } else { // the smallest block of at least 64 threads; one FP32 state 128 while the device has a block per SM
         // (1024^2 28.3 -> 24.5 us a step, 128^3 49.0 -> 47.0; FP64 and several states lose: 128^3 x 2 FP64 134 -> 139)
