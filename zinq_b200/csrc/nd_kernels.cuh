@@ -1198,12 +1198,13 @@ __device__ __forceinline__ void cta_partials(const double (&a)[NV], uint32_t act
 // The stage holds element t of line g at t W + g, as the box lands.
 // TM_KOBS (the momentum observables of phi after its forward transform along axis 0) stores
 // nothing: its sums run over the CTA's tiles and are written once, at column blockIdx.x.
-// TM_SCALE (the first tile pass of an imaginary-time step): every CTA sums the norm's partials of the
+// SCALE (TM_SCALE: the first tile pass of an imaginary-time step; a form of its own, since the code costs the others
+// 3-6 % of a step, 32^3 x 2 FP64 18.2 -> 19.3 us): every CTA sums the norm's partials of the
 // row launch before it, in the same order, while its first tile is on the way, and normalises what it
 // loads.  Scaling later (in the row pass that closes the step, where the sum is known anyway) would let
 // two steps' factors exp(-E dt) act on the state before it is normalised, which FP32 does not hold for
 // wells far from the zero of energy.
-template <typename T, int D, int LOGN>
+template <typename T, int D, int LOGN, bool SCALE>
 __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     nd_tile_tma_kernel(const __grid_constant__ NdJob<T> J, const __grid_constant__ CUtensorMap map, const NdTma P,
                        size_t part_base, const __grid_constant__ NdFin F) {
@@ -1250,13 +1251,18 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
     // the first load overlaps the twiddle staging (the stage and the twiddles do not overlap)
     if (tid == 0 && !P.withhold) issue(blockIdx.x);
     for (int t = tid; t < PL::ntw; t += blockDim.x) tw[t] = J.twd[t];
-    __shared__ double norm_sum;
-    if ((P.mode & TM_SCALE) && tid < 32) {
-        const double x = warp_sum_partials(J.part, J.nparts, 0, P.ncols, Slots<D, 1>::norm);
-        if (tid == 0) norm_sum = x;
+    double nf = 1.0;
+    if constexpr (SCALE) {
+        __shared__ double norm_sum;
+        if (tid < 32) {
+            const double x = warp_sum_partials(J.part, J.nparts, 0, P.ncols, Slots<D, 1>::norm);
+            if (tid == 0) norm_sum = x;
+        }
+        __syncthreads();
+        nf = nd_norm_factor(norm_sum, J.dr);
+    } else {
+        __syncthreads();
     }
-    __syncthreads();
-    const double nf = (P.mode & TM_SCALE) ? nd_norm_factor(norm_sum, J.dr) : 1.0;
     // the thread's line g of the tile and its place i in the line: a warp takes whole lines where
     // they are short enough, neighbouring threads neighbouring lines
     constexpr bool WARP = TPL <= 32;
@@ -1283,7 +1289,7 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
         if (ok) {
 #pragma unroll
             for (int t = 0; t < 16; ++t) v[t] = stage[((i + t * TPL) << logW) + g];
-            if (P.mode & TM_SCALE)
+            if constexpr (SCALE)
 #pragma unroll
                 for (int t = 0; t < 16; ++t) v[t] = nd_scaled<T>(v[t], nf);
         }
