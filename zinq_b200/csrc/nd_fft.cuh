@@ -61,6 +61,14 @@ template <typename T> __host__ __device__ inline int exch_stride(int logn, int s
     return ld;
 }
 
+// Tile passes: whether a warp takes whole lines (32 / TPL of them), with no CTA barrier at a transform's
+// boundaries.  Not where those lines' elements side by side are less than a 32-byte sector: from 512 points
+// (256 in FP32) up a warp's loads and stores at the axis stride would be part of a sector each.  There
+// neighbouring threads take the tile's neighbouring lines and the CTA waits at the boundaries.
+template <typename T> __host__ __device__ constexpr bool tile_warp_lines(int logn) {
+    return logn <= 9 && (512 >> logn) * sizeof(cx<T>) >= 32;
+}
+
 struct SyncWarp {
     __device__ __forceinline__ void operator()() const { __syncwarp(); }
 };

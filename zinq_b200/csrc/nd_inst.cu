@@ -114,7 +114,7 @@ inline int log2_of(int n) {
 // exchange line stride of the two passes (exch_stride): rows take consecutive threads; a tile's lines
 // sit side by side, as many as share a warp
 inline int row_ldx(int n) { return exch_stride<T>(log2_of(n), 0); }
-inline int tile_ldx(int n, int W) { return exch_stride<T>(log2_of(n), n <= 512 ? 512 / n : W); }
+inline int tile_ldx(int n, int W) { return exch_stride<T>(log2_of(n), tile_warp_lines<T>(log2_of(n)) ? 512 / n : W); }
 
 struct Launch {
     zqd_job* J;

@@ -1264,8 +1264,9 @@ __global__ void __launch_bounds__(LOGN == 12 ? 512 : 256, LOGN == 12 ? 1 : 2)
         __syncthreads();
     }
     // the thread's line g of the tile and its place i in the line: a warp takes whole lines where
-    // they are short enough, neighbouring threads neighbouring lines
-    constexpr bool WARP = TPL <= 32;
+    // that still puts lines of a 32-byte sector side by side (tile_warp_lines), neighbouring threads
+    // neighbouring lines
+    constexpr bool WARP = tile_warp_lines<T>(LOGN);
     constexpr int LPW = WARP ? 32 / TPL : 1;
     const int g = WARP ? (tid >> 5) * LPW + (tid & (LPW - 1)) : tid & (W - 1);
     const int i = WARP ? (tid & 31) / LPW : tid >> logW;
