@@ -684,6 +684,12 @@ struct Seq {
         ZQD_CUDA(cudaGetLastError());
         return ZQD_OK;
     }
+    // the row pass that opens a step by itself, with the absorbed sums of its first accumAbsorbed
+    int open(int s, bool track) {
+        const uint32_t mode = RM_RSTART | RM_FWD | RM_STORE;
+        if (!track) return Lc.row(mode, 0, Lc.R2);
+        return Lc.observe(mode, 0, Lc.R2, fin(s, 2, Lc.R2, Lc.R2 + Lc.row_cols, false, 0, nullptr, 0), false);
+    }
     int step(int s, int i) {
         const Opts& o = J->o;
         int rc;
@@ -703,6 +709,13 @@ struct Seq {
             const uint32_t o2 = obs | (defer ? (uint32_t)WM_NORM : 0u);
             return Lc.observe(mode, o2, Lc.R0, f, false, false, whist(s, i));
         }
+        const bool track = Lc.D.track;
+        if (!o.imag_nstate && !o.pot_td) { // stop_norm alone: close step i and observe it, decide, then open the next
+            const uint32_t mode = RM_OBS | RM_STORE | (i > 0 ? (uint32_t)(RM_INV | RM_REND) : 0u) | (needk ? (uint32_t)RM_PHI : 0u);
+            if ((rc = Lc.observe(mode, obs, Lc.R0, fin(s, 0, Lc.R0, Lc.R0 + Lc.row_cols, needk, mask, row, i), true, false, whist(s, i))))
+                return rc;
+            return i < iters ? open(s, track) : ZQD_OK;
+        }
         // Imaginary time, first state (nothing to orthogonalise against), no absorbing potential, after
         // step 0: the pass that closes step i also sums |psi|^2, and the next pass divides by the norm
         // as it loads psi, in place of the norm and normalisation kernels (quantum_dynamics.zig:898-906
@@ -719,7 +732,7 @@ struct Seq {
         // R0 holds the end-of-step sums of the row pass that closed step i (none at i = 0)
         const NdFin f = fin(s, 0, i > 0 ? Lc.R0 : Lc.R1, Lc.R1 + Lc.row_cols, needk, mask, row, i);
         // stop_norm decides before the next launch; tracked absorption's carry is replaced by that launch's sums
-        const bool track = Lc.D.track, now = f.has_stop || track;
+        const bool now = f.has_stop || track;
         if (fuse && !o.pot_td && i < iters) { // normalise, observe, and open step i+1 in one pass
             const uint32_t mode = RM_SCALE | RM_OBS | RM_RSTART | RM_FWD | RM_STORE | (needk ? (uint32_t)RM_PHI : 0u);
             return Lc.observe(mode, obs, Lc.R1, f, now, false, whist(s, i));
@@ -728,10 +741,7 @@ struct Seq {
         if ((rc = Lc.observe(omode, obs, Lc.R1, f, now, false, whist(s, i)))) return rc;
         if (i < iters) {
             if (o.pot_td && (rc = Lc.table(((double)i + 0.5) * o.time_step, 1))) return rc;
-            const uint32_t mode = RM_RSTART | RM_FWD | RM_STORE;
-            if (!track) return Lc.row(mode, 0, Lc.R2);
-            // the absorbed sums of step i+1's first accumAbsorbed
-            return Lc.observe(mode, 0, Lc.R2, fin(s, 2, Lc.R2, Lc.R2 + Lc.row_cols, false, 0, nullptr, 0), false);
+            return open(s, track);
         }
         return ZQD_OK;
     }
