@@ -49,7 +49,8 @@ template <typename T> __global__ void scale_kernel(cx<T>* data, size_t N, double
 // line g at base + t stride + g on a strided axis (ROW = false), at base + g n + t on the last.  The
 // elements go from global memory to registers and back; only the boundaries between the radix passes
 // use shared memory.  A warp takes whole lines up to 512 points (32/TPL of them: four 16-byte or four
-// 8-byte lines side by side at 128 points, one or two sectors a row) and waits for no other warp; a
+// 8-byte lines side by side at 128 points, one or two sectors a row; one line at 512, a part of a sector) and
+// waits for no other warp; a
 // CTA takes W lines above.  The twiddles (under 2 KB at 128 points, 31 KB at 2048) are read through
 // L1: staging them would cost each short CTA a wait.  Against one line per CTA with 16-byte accesses at
 // the axis stride, 128^3 FP64 227 -> 49 us forward (with the caller's copy of the

@@ -501,7 +501,8 @@ int ZQD_ND_CREATE(zqd_job* J) {
     // columns of the partial sums: one per CTA of a row launch or of a momentum launch
     J->nd_row_cols = (int)(N / n / L);
     if (J->nd_row_tma) J->nd_row_cols = std::max(J->nd_row_phi_ctas, *std::max_element(J->nd_row_ctas, J->nd_row_ctas + RF_COUNT));
-    // a forced or tuned shape of the axis passes is theirs
+    // a forced or tuned shape of the axis passes is theirs (a table's entry for such a grid, also one written before the
+    // one-cluster kernel existed, keeps the axis passes; zqd_autotune writes one only where it beat that kernel)
     J->nd_small = J->d == 2 && J->nd_tma && J->nd_row_tma && log2_of(n) <= ND_SMALL_LOGN_MAX && !ov.rows && !ov.tile && !ov.tma_rows && !ov.tma_w;
     J->nd_k_cols = J->nd_tma ? J->nd_tma_ctas : (int)(S * (N / n / Tn));
     const size_t nparts = 3 * (size_t)J->nd_row_cols + J->nd_k_cols + 1024;

@@ -5,7 +5,8 @@
 // cluster: CTA c of the cluster owns the columns and the rows c n/C .. (c + 1) n/C, transforms its
 // columns (forward FFT, kinetic phase, inverse FFT), then its rows (inverse FFT, R, observables, R,
 // forward FFT), with a cluster barrier after each half.  The state goes between the halves through L2;
-// the tables a CTA reads every step stay in its L1.  The sums of a row wait in shared memory for a spare
+// what a CTA reads of the tables every step fits its L1 up to three states (128^2 x 4: R alone is 164 KB a CTA, read
+// from L2).  The sums of a row wait in shared memory for a spare
 // warp of CTA 0, which writes the observables row while the others transform the next step's columns.
 // 128^2 x 2 states FP64: 13.1 -> 9.6 us a step, 64^2 x 1: 11.0 -> 7.3.
 #pragma once

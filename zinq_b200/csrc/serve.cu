@@ -11,7 +11,8 @@
 // failure and cancellation are events too, and zqd_server_wait hands the result over.
 // 1-D single-solve requests whose line fits one CTA go to the persistent line-service kernel
 // instead (service.h): resident CTAs claim them from a table in pinned memory as they are posted
-// and publish every row; a poller thread streams those rows and completes the requests.
+// and publish their rows, no later than the pieces of stream_steps are complete; a poller thread streams
+// those rows and completes the requests.
 // The reference has no serving layer: this is the request loop around its quantum_dynamics.run.
 #include <algorithm>
 #include <atomic>
@@ -261,8 +262,6 @@ void zqd_server::run_active(std::vector<Req> group, cudaStream_t st) {
     const uint64_t key = group.front()->group_key;
     auto create = [&](const Req& q) -> bool {
         zqd::Opts o = q->o;
-        // several workers' jobs share the device: one resident CTA per SM for the persistent tile pass
-        o.tma_ctas_per_sm = 1;
         const int rc = zqd::job_create_opts(std::move(o), &q->job, st);
         if (rc) {
             finish(q, rc, zqd::last_error(), nullptr);
