@@ -240,10 +240,11 @@ int line_room_f4(const LaunchShape*, size_t*, size_t*);
 // reference does: the results differ by the roundings of that pair), and the ring of unreduced sums (up
 // to 16 steps and 64 KB; a single CTA 8 steps and 40 KB).  Both may go 10 KB beyond the budget of the tables,
 // to what the launch allows: the longest lines' tables leave less than a row below it, and their steps
-// would each be reduced at once (32768 points FP64 16.8 us a step, with three rows 15.8).  A ring of one
-// row pays on CTAs of up to 256 threads (8192 points x 4 states FP64 with energies 33.9 -> 31.5 us a
-// step), not where its traffic does not: rows above 16 KB want three (8192 x 4 FP32: 27.3 us reduced at
-// once, 29.3 with two rows).
+// would each be reduced at once (32768 points FP64 16.8 us a step, with three rows 15.8).  On CTAs of up to
+// 384 threads any ring pays (8192 points x 4 states FP64 with energies 33.9 us a step at once, 31.5 with
+// one row; 4096 x 3 FP64 with nine values 15.8 at once, 14.0 with two rows; 8192 x 3 FP32 with energies 31.9 and
+// 28.9), on larger ones two rows of up to 16 KB do and of larger rows three (8192 x 4 FP32: 27.3 at once,
+// 29.3 with two rows of 32 KB).
 // The service kernel takes the same buffer and as many of the ring's rows as leave its CTAs their places; a
 // row's sums do not depend on how many wait.
 static int line_extra_smem(zqd_job* J, size_t budget) {
@@ -275,7 +276,7 @@ static int line_extra_smem(zqd_job* J, size_t budget) {
     const size_t most = std::min<size_t>(J->C > 1 ? 64 * 1024 : 40 * 1024, room > J->smem ? room - J->smem : 0);
     const size_t want = J->C > 1 ? RING_STEPS : RING_STEPS / 2, steps = step ? std::min(want, most / step) : want;
     // stop_norm needs each step's norm at once
-    if (steps >= (step > 16384 ? 3u : J->threads > 256 ? 2u : 1u) && J->smem + step <= svc && !(o.has_cap && o.cap_has_stop)) {
+    if (steps >= (J->threads < 512 ? 1u : step <= 16384 ? 2u : 3u) && J->smem + step <= svc && !(o.has_cap && o.cap_has_stop)) {
         J->ring_off = (int)J->smem;
         J->ring_steps = (int)steps;
         J->ring_service = (int)(step ? std::min(steps, (svc - J->smem) / step) : steps);
