@@ -112,7 +112,7 @@ inline int log2_of(int n) {
     return l;
 }
 // exchange line stride of the two passes (exch_stride): rows take consecutive threads; a tile's lines
-// sit side by side, as many as share a warp
+// sit side by side, those of a warp (tile_warp_lines) or all
 inline int row_ldx(int n) { return exch_stride<T>(log2_of(n), 0); }
 inline int tile_ldx(int n, int W) { return exch_stride<T>(log2_of(n), tile_warp_lines<T>(log2_of(n)) ? 512 / n : W); }
 
@@ -317,7 +317,7 @@ inline bool tuned_threads_ok(size_t points, size_t most) { return points / 8 % 3
 
 // The TMA-staged tile pass: lines per tile W (a power of two, W <= n) with rows of W c >= 16
 // bytes (an even number of 8-byte words), W n / 16 threads (whole warps, at most 256, 512 on lines of
-// 4096 points; a line of at most 512 points within one warp) and the stage, exchange and
+// 4096 points) and the stage, exchange and
 // twiddles within the shared-memory budget; by default the widest W up to 64-byte rows.  w_override
 // (the autotuner's candidate or table entry): 0 keeps the default, -1 keeps the earlier tile
 // kernel, else W.  ZQD_ND_TMA=0 in the environment also keeps it.
