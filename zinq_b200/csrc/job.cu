@@ -764,10 +764,15 @@ template <typename T> static int fetch_line(zqd_job* J, zqd_result* R) {
         const size_t n = (size_t)J->n, m = (size_t)J->m, C = (size_t)J->C;
         auto put = [&](size_t first, size_t cnt, const cx<T>* z) {
             if (J->d == 1) { // un-permute: position p = c*m + j of a state holds grid index c + C*j
-                for (size_t e = 0; e < cnt; ++e) {
-                    const size_t st = (first + e) / n, p = (first + e) - st * n, c = p / m, j = p - c * m, x = c + C * j;
-                    dst[2 * (st * n + x)] = (double)z[e].x;
-                    dst[2 * (st * n + x) + 1] = (double)z[e].y;
+                size_t st = first / n, p = first - st * n, c = p / m, j = p - c * m;
+                for (size_t e = 0; e < cnt;) {
+                    double* to = dst + 2 * (st * n + c); // grid indices c + C j, counted up without a division a point
+                    for (; j < m && e < cnt; ++j, ++e) {
+                        to[2 * C * j] = (double)z[e].x;
+                        to[2 * C * j + 1] = (double)z[e].y;
+                    }
+                    j = 0;
+                    if (++c == C) c = 0, ++st;
                 }
             } else if (sizeof(T) == 8) {
                 std::memcpy(dst + 2 * first, z, cnt * sizeof(cx<T>));
